@@ -873,7 +873,8 @@ int Batch::build_group(Group &g, const int *const *rp, const int *const *ci,
     return e;
   if (int e = tmp.get(&fb_d, 1))
     return e;
-  if (int e = fsai_build_values(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fb_d, 0))
+  if (int e = fsai_build_values(n, fsai_max_pattern(g_rp), a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d,
+                                fb_d, 0))
     return e;
   const int blocks = (int)std::min<long long>(((long long)nnz_g + 255) / 256, 148LL * 16);
   b_scatter_kernel<<<std::max(blocks, 1), 256>>>(gt_v_d, t_of_d, g_v_d, (long long)nnz_g);

@@ -14,9 +14,8 @@
 // while holding ~5% fewer non-zeros, and it is built in milliseconds instead
 // of seconds.
 //
-// One warp per row: lanes gather the |P_i| x |P_i| local matrix (|P_i| <= 32)
-// into shared memory, factor it (Cholesky) and back-substitute.  FP64
-// throughout.  A local matrix that is not positive definite (indefinite A)
+// A group of lanes per row gathers the |P_i| x |P_i| local matrix (|P_i| <=
+// 32), factors it (L D L^T) and back-substitutes.  FP64 throughout.  A local matrix that is not positive definite (indefinite A)
 // falls back to the Jacobi row e_i / sqrt(a_ii) when a_ii > 0, else to e_i,
 // and is counted.
 #include <cuda_runtime.h>
@@ -31,89 +30,165 @@
 namespace ispm {
 namespace {
 
-constexpr int kWarpsPerBlock = 4;  // 4 x 32 x 33 doubles = 33.8 KB of shared memory
+constexpr int kWarpsPerBlock = 4;
 constexpr int kMaxPattern = 32;
 
+// One factor row per group of G lanes (G = 4, 8, 16 or 32, the smallest that
+// holds the longest pattern), 32 / G rows a warp; lane l owns row l of the
+// local matrix in registers.
+//
+// What bounds it: shared-memory and L1 wavefronts (83% of their rate on the
+// 72^3 27-point matrix, issue slots 67%, DRAM 4%).  A row of that stencil (K =
+// 14) needs about 110 FP64 multiply-adds a lane fed by shared-memory
+// broadcasts, and its 14 x 14 local matrix comes from 14 rows of A that
+// neighbouring factor rows share through L1; the bytes (12 per entry of A, 8
+// per entry of G) are a fraction of that time.  373,248 rows take 0.46 ms;
+// one warp a row with a walk per lane, a Cholesky factorization in shared
+// memory and a serial back-substitution took 3.39 ms.  So:
+//  * the group reads each row of A it needs as one coalesced run (the entries
+//    from the diagonal on, the half the factorization uses) and finds their
+//    places in the pattern by a binary search in shared memory, instead of a
+//    lane walking a whole row entry by entry;
+//  * L D L^T without square roots: column k goes once through shared memory
+//    (unscaled), every lane updates its own row from broadcast reads, and one
+//    reciprocal serves the column;
+//  * the last row of L^-1, z = L^-T e, is all that the factor row needs
+//    (g = z / sqrt(d_last)): one lane-parallel back-substitution, reading the
+//    stored columns.
+template <int G>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     fsai_rows_kernel(int n, const int *__restrict__ a_rp, const int *__restrict__ a_ci,
                      const double *__restrict__ a_v, const int *__restrict__ g_rp,
                      double *__restrict__ g_v, unsigned *fallbacks)
 {
-  __shared__ double sm[kWarpsPerBlock][kMaxPattern][kMaxPattern + 1];
-  __shared__ int pat[kWarpsPerBlock][kMaxPattern];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double(*L)[kMaxPattern + 1] = sm[w];
-  const int i = blockIdx.x * kWarpsPerBlock + w;
-  if (i >= n)
-    return;  // whole warp leaves together
-  const int g0 = g_rp[i], K = g_rp[i + 1] - g0;  // pattern = first K entries of row i
-  const int a0 = a_rp[i];
-  if (lane < K)
-    pat[w][lane] = __ldg(a_ci + a0 + lane);
-  __syncwarp();
-  // Lane l gathers column l of A[P,P]: entries a(p_l, p_k), k < K, by merging
-  // the (sorted) row p_l of A with the (sorted) pattern.
+  constexpr int R = 32 / G;   // rows a warp
+  constexpr int LD = G + 2;   // row length: even (16-byte reads), rows on distinct banks
+  constexpr int B = G < 8 ? G : 8;  // pattern rows whose loads are in flight together
+  constexpr int kNone = 0x7fffffff;
+  __shared__ __align__(16) double sm[kWarpsPerBlock * R][G][LD];
+  __shared__ int pats[kWarpsPerBlock * R][G];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & (G - 1), grp = threadIdx.x / G;
+  double(*S)[LD] = sm[grp];
+  int *pat = pats[grp];
+  const long long row = (long long)blockIdx.x * (kWarpsPerBlock * R) + grp;
+  const bool live = row < n;  // a group past the end keeps its warp company with K = 0
+  const int i = live ? (int)row : 0;
+  const int g0 = live ? __ldg(g_rp + i) : 0;
+  const int K = live ? __ldg(g_rp + i + 1) - g0 : 0;  // pattern = first K entries of row i
+  const int kw = __reduce_max_sync(full, K);
+  const int p = lane < K ? __ldg(a_ci + __ldg(a_rp + i) + lane) : kNone;
+  pat[lane] = p;
+  // row p of A from its diagonal on
+  int start = 0, stop = 0;
   if (lane < K) {
-    const int row = pat[w][lane];
-    int e = __ldg(a_rp + row);
-    const int stop = __ldg(a_rp + row + 1);
-    for (int k = 0; k < K; k++) {
-      const int want = pat[w][k];
-      while (e < stop && __ldg(a_ci + e) < want)
-        e++;
-      L[k][lane] = (e < stop && __ldg(a_ci + e) == want) ? __ldg(a_v + e) : 0.0;
+    start = __ldg(a_rp + p) + (__ldg(g_rp + p + 1) - __ldg(g_rp + p)) - 1;
+    stop = __ldg(a_rp + p + 1);
+  }
+#pragma unroll
+  for (int k = 0; k < G; k += 2)
+    *reinterpret_cast<double2 *>(&S[lane][k]) = make_double2(0.0, 0.0);
+  __syncwarp();
+  // S[r][c] = a(p_c, p_r), r >= c
+  for (int c0 = 0; c0 < kw; c0 += B) {
+    int col[B];
+    double val[B];
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+      const int e = __shfl_sync(full, start, c0 + q, G) + lane;
+      const bool in = e < __shfl_sync(full, stop, c0 + q, G);
+      col[q] = in ? __ldg(a_ci + e) : kNone;
+      val[q] = in ? __ldg(a_v + e) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+      int e = __shfl_sync(full, start, c0 + q, G) + lane;
+      const int end = __shfl_sync(full, stop, c0 + q, G);
+      for (;;) {
+        if (col[q] <= i) {
+          int at = 0;
+#pragma unroll
+          for (int s = G / 2; s > 0; s >>= 1)
+            at = pat[at + s] <= col[q] ? at + s : at;
+          if (pat[at] == col[q])
+            S[at][c0 + q] = val[q];
+        }
+        // a longer run: on while its last entry is still left of column i
+        if (!__any_sync(full, lane == G - 1 && col[q] < i))
+          break;
+        e += G;
+        const bool in = col[q] < i && e < end;
+        col[q] = in ? __ldg(a_ci + e) : kNone;
+        val[q] = in ? __ldg(a_v + e) : 0.0;
+      }
     }
   }
   __syncwarp();
-  // Cholesky, right-looking, lower triangle; lane j owns column j.
+  double a[G];
+#pragma unroll
+  for (int k = 0; k < G; k += 2) {
+    const double2 v = *reinterpret_cast<const double2 *>(&S[lane][k]);
+    a[k] = v.x;
+    a[k + 1] = v.y;
+  }
+  if (lane >= K) {  // identity past the pattern
+#pragma unroll
+    for (int k = 0; k < G; k++)
+      a[k] = k == lane ? 1.0 : 0.0;
+  }
+  __syncwarp();
   bool ok = true;
-  for (int k = 0; k < K; k++) {
-    const double d = L[k][k];
-    if (!(d > 0.0)) {
-      ok = false;
-      break;  // uniform: every lane reads the same shared value
+  double rd_own = 1.0, d_own = 1.0;
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    if (k < kw) {
+      S[k][lane] = a[k];  // column k, unscaled (the lanes k .. are read)
+      __syncwarp();
+      const double d = S[k][k];
+      ok = ok && d > 0.0;
+      const double rd = 1.0 / d;
+      if (lane == k) {
+        rd_own = rd;
+        d_own = d;
+      }
+      const double l = a[k] * rd;
+#pragma unroll
+      for (int j = k + 1; j < G; j++)
+        a[j] = fma(-l, S[k][j], a[j]);
     }
-    const double lkk = sqrt(d);
-    __syncwarp();
-    if (lane == k)
-      L[k][k] = lkk;
-    if (lane > k && lane < K)
-      L[lane][k] /= lkk;
-    __syncwarp();
-    // trailing update of column j = lane (rows i >= j)
-    if (lane > k && lane < K) {
-      const double ljk = L[lane][k];
-      for (int r = lane; r < K; r++)
-        L[r][lane] -= L[r][k] * ljk;
-    }
-    __syncwarp();
   }
-  if (!ok) {
-    // Jacobi fallback on the diagonal entry (the last pattern slot is i)
-    if (lane == 0) {
-      const double aii = __ldg(a_v + a0 + K - 1);
-      atomicAdd(fallbacks, 1u);
-      for (int k = 0; k < K - 1; k++)
-        g_v[g0 + k] = 0.0;
-      g_v[g0 + K - 1] = aii > 0.0 ? 1.0 / sqrt(aii) : 1.0;
+  __syncwarp();
+  double s = 0.0, z = lane == K - 1 ? 1.0 : 0.0;
+#pragma unroll
+  for (int c = G - 1; c > 0; c--) {
+    if (c < kw) {
+      const double zc = __shfl_sync(full, z, c, G);
+      s = fma(S[lane][c], zc, s);  // used by the lanes left of c alone
+      if (lane == c - 1 && c < K)
+        z = -rd_own * s;
     }
-    return;
   }
-  // L L^T y = e_{K-1}: y_{K-1} = 1 / L_{K-1,K-1}^2, then back-substitute;
-  // g = y / sqrt(y_{K-1}) = y * L_{K-1,K-1}.  Sequential in lane 0 (K <= 32).
-  if (lane == 0) {
-    double y[kMaxPattern];
-    const double lnn = L[K - 1][K - 1];
-    y[K - 1] = 1.0 / (lnn * lnn);
-    for (int r = K - 2; r >= 0; r--) {
-      double s = 0.0;
-      for (int c = r + 1; c < K; c++)
-        s = fma(L[c][r], y[c], s);
-      y[r] = -s / L[r][r];
+  const double dl = __shfl_sync(full, d_own, K > 0 ? K - 1 : 0, G);
+  if (lane < K) {
+    double g = z / sqrt(dl);
+    if (!ok) {
+      // Jacobi row on the diagonal entry (the last pattern slot is i)
+      const double aii = __ldg(a_v + __ldg(a_rp + i) + K - 1);
+      g = lane < K - 1 ? 0.0 : aii > 0.0 ? 1.0 / sqrt(aii) : 1.0;
+      if (lane == 0)
+        atomicAdd(fallbacks, 1u);
     }
-    for (int k = 0; k < K; k++)
-      g_v[g0 + k] = y[k] * lnn;
+    g_v[g0 + lane] = g;
   }
+}
+
+template <int G>
+void launch_rows(int n, const int *a_rp, const int *a_ci, const double *a_v, const int *g_rp,
+                 double *g_v, unsigned *fb, cudaStream_t s)
+{
+  const int rows = kWarpsPerBlock * (32 / G);
+  fsai_rows_kernel<G><<<(n + rows - 1) / rows, kWarpsPerBlock * 32, 0, s>>>(n, a_rp, a_ci, a_v,
+                                                                            g_rp, g_v, fb);
 }
 
 }  // namespace
@@ -165,12 +240,29 @@ void fsai_transpose_pattern(int n, const std::vector<int> &g_rp, const std::vect
     }
 }
 
-int fsai_build_values(int n, const int *a_rp_d, const int *a_ci_d, const double *a_v_d,
-                      const int *g_rp_d, double *g_v_d, unsigned *fallbacks_d, cudaStream_t s)
+int fsai_max_pattern(const std::vector<int> &g_rp)
 {
-  const int blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  fsai_rows_kernel<<<blocks, kWarpsPerBlock * 32, 0, s>>>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d,
-                                                          g_v_d, fallbacks_d);
+  int k = 0;
+  for (size_t i = 0; i + 1 < g_rp.size(); i++)
+    k = std::max(k, g_rp[i + 1] - g_rp[i]);
+  return k;
+}
+
+int fsai_build_values(int n, int max_pattern, const int *a_rp_d, const int *a_ci_d,
+                      const double *a_v_d, const int *g_rp_d, double *g_v_d,
+                      unsigned *fallbacks_d, cudaStream_t s)
+{
+  if (max_pattern > kMaxPattern)
+    return fail(ISPM_ERR_INVALID, "FSAI pattern of %d entries (at most %d)", max_pattern,
+                kMaxPattern);
+  if (max_pattern <= 4)
+    launch_rows<4>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
+  else if (max_pattern <= 8)
+    launch_rows<8>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
+  else if (max_pattern <= 16)
+    launch_rows<16>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
+  else
+    launch_rows<32>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
   cudaError_t e = cudaPeekAtLastError();
   return e == cudaSuccess ? ISPM_OK : fail(ISPM_ERR_CUDA, "fsai rows: %s", cudaGetErrorString(e));
 }
@@ -241,7 +333,7 @@ extern "C" int ispm_fsai_sym_gpu(int out_dtype, int n, const int *row_ptr, const
   if (int e = mem.get(&fb, 1))
     return e;
   ISPM_CUDA_TRY(cudaMemset(fb, 0, sizeof(unsigned)));
-  if (int e = fsai_build_values(n, a_rp, a_ci, a_v, gr, g_v, fb, 0))
+  if (int e = fsai_build_values(n, fsai_max_pattern(g_rp), a_rp, a_ci, a_v, gr, g_v, fb, 0))
     return e;
   std::vector<double> gv(nnz_g);
   ISPM_CUDA_TRY(cudaMemcpy(gv.data(), g_v, nnz_g * sizeof(double), cudaMemcpyDeviceToHost));

@@ -585,6 +585,7 @@ struct Solver {
     unsigned *t_of = nullptr, *pos_g = nullptr, *pos_t = nullptr, *fb = nullptr;
     double *g_v = nullptr, *gt_v = nullptr;
     long long nnz_g = 0;
+    int max_pattern = 0;
     bool f16 = false;
   } fsai;
   bool fsai_kept = false;
@@ -1030,7 +1031,7 @@ template <class T> int to_device(DevMem &mem, T **d, const T *h, size_t count)
 // factor matrices through their CSR-entry -> slot maps (legacy stream).
 int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
 {
-  if (int e = fsai_build_values(S.n, f.a_rp, f.a_ci, a_v, f.g_rp, f.g_v, f.fb, 0))
+  if (int e = fsai_build_values(S.n, f.max_pattern, f.a_rp, f.a_ci, a_v, f.g_rp, f.g_v, f.fb, 0))
     return e;
   const int blocks = grid_for(f.nnz_g);
   scatter_kernel<<<blocks, kThreads>>>(f.gt_v, f.t_of, f.g_v, f.nnz_g);
@@ -1105,6 +1106,7 @@ int build_fsai_on_device(Solver &S, int n, const int *rp, const int *ci, const d
   DevMem &mem = S.refreshable ? S.mem : tmp;
   Solver::FsaiArrays f;
   f.nnz_g = (long long)nnz_g;
+  f.max_pattern = fsai_max_pattern(g_rp);
   f.f16 = f16;
   double *a_v_d;
   if (int e = to_device(mem, &f.a_rp, rp, (size_t)n + 1))
