@@ -48,6 +48,7 @@
 #include "fsai.h"
 #include "nvtx_range.h"
 #include "operator.h"
+#include "persist.h"
 
 namespace ispm {
 namespace {
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(kThreads)
     b_update_kernel(const T *__restrict__ p, const T *__restrict__ q, T *__restrict__ r,
                     T *__restrict__ d, LaneArgs la, int par)
 {
+  pdl_wait();
   const int t = blockIdx.x;
   const int L = la.tile_lane[t];
   if (la.state[L] != kRun)
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(kThreads)
     st4(r + i, rv);
     st4(d + i, dv);
   }
+  pdl_trigger();
   if (lane_finish(acc, la.part_rr, la.t_rr, la.rr, L, la.lane_tile0[L], la.lane_ntile[L], ok) &&
       ok)
     la.it[L] += 1;
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(kThreads)
     b_direction_kernel(const T *__restrict__ z, T *__restrict__ p, LaneArgs la,
                        const double *__restrict__ rz_lane, int par, int mode)
 {
+  pdl_wait();
   const int t = blockIdx.x;
   const int L = la.tile_lane[t];
   if (la.state[L] != kRun)
@@ -228,6 +232,7 @@ __global__ void __launch_bounds__(kThreads)
       pv.v[k] = fma(b, pv.v[k], zv.v[k]);
   }
   st4(p + i, pv);
+  pdl_trigger();
   if (lead) {
     la.rz_cur[L] = rzn;
     if (mode == 0) {
@@ -413,6 +418,18 @@ struct Batch {
   int chunk = 16;
   int graph_nodes = 0;  // kernels in one replay of the chunk graph
   int launches = 0;  // kernels launched by the last solve (graph nodes counted)
+  // one cooperative launch a solve (persist.cu) for batches that fit L2
+  struct Persist {
+    bool on = false;
+    PersistParams prm;
+    PersistKind kind;
+    std::vector<int> order;  // lane of each slot
+    int ctas = 0, threads = 256;
+    char *zero = nullptr;  // abort flag, a count per lane
+    size_t zero_bytes = 0;
+    PersistOut *host = nullptr;
+    unsigned *abort_h = nullptr;
+  } pk;
   bool completed = false;  // the last solve ran to its end (lane results are valid)
   bool verbose = getenv("ISPM_SOLVER_VERBOSE") && atoi(getenv("ISPM_SOLVER_VERBOSE")) > 0;
 
@@ -421,7 +438,7 @@ struct Batch {
     if (graph)
       cudaGraphExecDestroy(graph);
     for (void *p : {(void *)ib_h, (void *)res_h, (void *)rr_h, (void *)thr_h, (void *)ref_h,
-                    (void *)hb, (void *)hx})
+                    (void *)hb, (void *)hx, (void *)pk.host, (void *)pk.abort_h})
       if (p)
         cudaFreeHost(p);
     if (ev_in)
@@ -457,6 +474,7 @@ struct Batch {
   // q = A p (lane sums of p.q), every group.
   int spmv_a(cudaStream_t s)
   {
+    std::vector<LaneOp> ops;
     for (const Group &g : groups) {
       SpmvLanes ln = lanes_for(g, la.skip);
       ln.v = vp(P, g.row0);
@@ -465,11 +483,9 @@ struct Batch {
       ln.ticket = t_pq;
       ln.cta_beg = a_beg;
       ln.cta_cnt = a_cnt;
-      if (int e = g.Ain.apply_lanes(inner, vp(P, g.row0), vp(Q, g.row0), s, ln))
-        return e;
-      launches++;
+      ops.push_back(g.Ain.lane_op(vp(P, g.row0), vp(Q, g.row0), ln));
     }
-    return ISPM_OK;
+    return launch_spmv_lanes(inner, ops.data(), (int)ops.size(), s, true, &launches);
   }
 
   // z = G^T (G r) (lane sums of r.z); nothing without a preconditioner.
@@ -477,21 +493,21 @@ struct Batch {
   {
     if (!have_prec)
       return ISPM_OK;
+    std::vector<LaneOp> ops, opt;
     for (const Group &g : groups) {
       SpmvLanes ln = lanes_for(g, la.skip);
-      if (int e = g.G.apply_lanes(inner, vp(R, g.row0), vp(TT, g.row0), s, ln))
-        return e;
+      ops.push_back(g.G.lane_op(vp(R, g.row0), vp(TT, g.row0), ln));
       ln.v = vp(R, g.row0);
       ln.out = la.rzn;
       ln.part = part_h;
       ln.ticket = t_rz;
       ln.cta_beg = h_beg;
       ln.cta_cnt = h_cnt;
-      if (int e = g.Ht.apply_lanes(inner, vp(TT, g.row0), vp(Z, g.row0), s, ln))
-        return e;
-      launches += 2;
+      opt.push_back(g.Ht.lane_op(vp(TT, g.row0), vp(Z, g.row0), ln));
     }
-    return ISPM_OK;
+    if (int e = launch_spmv_lanes(inner, ops.data(), (int)ops.size(), s, true, &launches))
+      return e;
+    return launch_spmv_lanes(inner, opt.data(), (int)opt.size(), s, true, &launches);
   }
 
   // One iteration; `last` (the chunk's final step) stops after the r / d
@@ -501,8 +517,9 @@ struct Batch {
   {
     if (int e = spmv_a(s))
       return e;
-    b_update_kernel<T><<<n_tiles, kThreads, 0, s>>>((const T *)vec[P], (const T *)vec[Q],
-                                                    (T *)vec[R], (T *)vec[D], la, par);
+    ISPM_CUDA_TRY(launch_kernel(b_update_kernel<T>, dim3(n_tiles), dim3(kThreads), 0, s, true,
+                                (const T *)vec[P], (const T *)vec[Q], (T *)vec[R], (T *)vec[D],
+                                la, par));
     if (int e = launched("batch update"))
       return e;
     if (last)
@@ -510,8 +527,9 @@ struct Batch {
     if (int e = precondition(s))
       return e;
     const T *z = (const T *)(have_prec ? vec[Z] : vec[R]);
-    b_direction_kernel<T><<<n_tiles, kThreads, 0, s>>>(z, (T *)vec[P], la,
-                                                       have_prec ? la.rzn : la.rr, par, 0);
+    ISPM_CUDA_TRY(launch_kernel(b_direction_kernel<T>, dim3(n_tiles), dim3(kThreads), 0, s, true,
+                                z, (T *)vec[P], la,
+                                (const double *)(have_prec ? la.rzn : la.rr), par, 0));
     return launched("batch direction");
   }
 
@@ -561,12 +579,11 @@ struct Batch {
       b_fold_kernel<T><<<n_tiles, kThreads, 0, s>>>(x, (T *)vec[D], la);
       if (int e = launched("batch fold"))
         return e;
-      for (const Group &g : groups) {
-        SpmvLanes ln = lanes_for(g, la.fin);
-        if (int e = g.A64.apply_lanes(ISPM_F64, x + g.row0, t64 + g.row0, s, ln))
-          return e;
-        launches++;
-      }
+      std::vector<LaneOp> ops;
+      for (const Group &g : groups)
+        ops.push_back(g.A64.lane_op(x + g.row0, t64 + g.row0, lanes_for(g, la.fin)));
+      if (int e = launch_spmv_lanes(ISPM_F64, ops.data(), (int)ops.size(), s, false, &launches))
+        return e;
     }
     b_residual_kernel<T><<<n_tiles, kThreads, 0, s>>>(b, zero_x ? nullptr : t64, r64,
                                                       (T *)vec[R], la);
@@ -610,20 +627,45 @@ struct Batch {
     return inner == ISPM_F32 ? restart_t<float>(s) : restart_t<double>(s);
   }
 
-  int solve(const double *b, double *x, ispm_solve_stats *lane_stats, ispm_solve_stats *total,
-            cudaStream_t s)
+  int init_persist();
+
+  // The whole batch in one launch; fills the lane results.
+  int run_persistent(const double *b, double *x, cudaStream_t s)
   {
-    auto t0 = std::chrono::steady_clock::now();
-    launches = 0;
-    completed = false;
+    Persist &k = pk;
+    k.prm.b = b;
+    k.prm.x = x;
+    ISPM_CUDA_TRY(cudaMemsetAsync(k.zero, 0, k.zero_bytes, s));
+    if (int e = persist_launch(k.prm, k.kind, k.ctas, k.threads, s))
+      return e;
+    launches = 1;
+    ISPM_CUDA_TRY(cudaMemcpyAsync(k.host, k.prm.out, sizeof(PersistOut) * n_lanes,
+                                  cudaMemcpyDeviceToHost, s));
+    ISPM_CUDA_TRY(cudaMemcpyAsync(k.abort_h, k.prm.abort, sizeof(unsigned),
+                                  cudaMemcpyDeviceToHost, s));
+    ISPM_CUDA_TRY(cudaStreamSynchronize(s));
+    if (*k.abort_h)
+      return fail(ISPM_ERR_TIMEOUT, "persistent batch: a group of CTAs waited too long");
+    for (int slot = 0; slot < n_lanes; slot++) {
+      const PersistOut &o = k.host[slot];
+      const int L = k.order[slot];
+      rel[L] = o.rel;
+      status[L] = o.status;
+      refinements[L] = o.replacements;
+      restarts[L] = o.restarts;
+      ib_h[4 * n_lanes + L] = o.iterations;
+    }
+    if (verbose)
+      fprintf(stderr, "[ispm batch] one launch, %d CTAs\n", k.ctas);
+    return ISPM_OK;
+  }
+
+  // Chunks of iterations for all lanes in lockstep, a reliable update after each.
+  int run_chunks(const double *b, double *x, cudaStream_t s)
+  {
     const int n = n_lanes;
     int *state = ib_h, *skip = ib_h + n, *fin = ib_h + 2 * n, *fresh = ib_h + 3 * n,
         *its = ib_h + 4 * n;
-    bnorm.assign(n, 0.0);
-    rel.assign(n, 0.0);
-    refinements.assign(n, 0);
-    restarts.assign(n, 0);
-    status.assign(n, ISPM_OK);
     for (int L = 0; L < n; L++)
       state[L] = kRun, skip[L] = 0, fin[L] = 0, fresh[L] = 1, its[L] = 0;
     ISPM_CUDA_TRY(cudaMemcpyAsync(ib, ib_h, 5 * sizeof(int) * n, cudaMemcpyHostToDevice, s));
@@ -704,6 +746,24 @@ struct Batch {
       if (verbose)
         fprintf(stderr, "[ispm batch] round %d: %d of %d lanes continue\n", rounds, active, n);
     }
+    return ISPM_OK;
+  }
+
+  int solve(const double *b, double *x, ispm_solve_stats *lane_stats, ispm_solve_stats *total,
+            cudaStream_t s)
+  {
+    auto t0 = std::chrono::steady_clock::now();
+    launches = 0;
+    completed = false;
+    const int n = n_lanes;
+    int *its = ib_h + 4 * n;
+    bnorm.assign(n, 0.0);
+    rel.assign(n, 0.0);
+    refinements.assign(n, 0);
+    restarts.assign(n, 0);
+    status.assign(n, ISPM_OK);
+    if (int e = pk.on ? run_persistent(b, x, s) : run_chunks(b, x, s))
+      return e;
     int worst = ISPM_OK, max_it = 0, max_ref = 0, all_conv = 1;
     double max_rel = 0.0;
     for (int L = 0; L < n; L++) {
@@ -764,6 +824,107 @@ struct Batch {
             const double *const *v, const int *n_rhs);
   int build_group(Group &g, const int *const *rp, const int *const *ci, const double *const *v);
 };
+
+// Decide whether solves run as one cooperative launch (persist.cu), and
+// prepare it: what an iteration reads fits L2 with room to spare.  16 systems
+// of 12 to 40 a side, 41 lanes: 1.86 against 3.04 ms with the shared launches.
+// A larger batch keeps those, whose lanes read a system's matrix tile one
+// after another out of L2.
+int Batch::init_persist()
+{
+  Persist &k = pk;
+  double bytes = 6.0 * esize() * n_stack;
+  std::vector<PersistLane> pl((size_t)n_lanes);
+  std::vector<double> work((size_t)n_lanes);
+  unsigned low = ~0u;
+  for (const Group &g : groups) {
+    bytes += (double)g.Ain.bytes();
+    low = std::min(low, g.Ain.dev.meta.slice_height);
+    if (have_prec) {
+      bytes += (double)g.G.bytes() + (double)g.Ht.bytes();
+      low = std::min({low, g.G.dev.meta.slice_height, g.Ht.dev.meta.slice_height});
+    }
+    // the group's mean entries a row, inner matrix and factors
+    const double wide = ((double)g.Ain.dev.meta.n_elms +
+                         (have_prec ? (double)g.G.dev.meta.n_elms + g.Ht.dev.meta.n_elms : 0.0)) /
+                        std::max(1.0, (double)g.mat_tiles * kTile);
+    for (size_t i = 0; i < g.systems.size(); i++) {
+      const int sys = g.systems[i];
+      const long long m0 = (long long)g.sys_tile0[i] * kTile;
+      for (int L = (int)sys_lane0[sys]; L < (int)sys_lane0[sys] + sys_rhs[sys]; L++) {
+        PersistLane &l = pl[L];
+        if (!persist_op(g.Ain, m0, l.A) || !persist_op(g.A64, m0, l.A64) ||
+            (have_prec && (!persist_op(g.G, m0, l.G) || !persist_op(g.Ht, m0, l.Ht))))
+          return ISPM_OK;
+        l.row0 = lanes[L].row0;
+        l.rows = l.n = lanes[L].ntile * kTile;
+        work[L] = (double)l.rows * (wide + 6.0);
+      }
+    }
+  }
+  if (bytes > kPersistMaxBatchBytes)
+    return ISPM_OK;
+  int most = 0;
+  k.kind.inner = inner;
+  k.kind.shape = persist_shape((double)n_stack, (double)device_sm_count() * 1024, 4.0, low);
+  if (int e = persist_capacity(k.kind, k.threads, 1, most))
+    return e;
+  if (most < 1)
+    return ISPM_OK;
+  std::vector<int> cta_lane, lane_count;
+  k.ctas = persist_assign(pl, work, most, k.order, cta_lane, lane_count);
+  std::vector<PersistLane> sorted;
+  k.prm.max_tiles = 1;
+  for (int L : k.order) {
+    sorted.push_back(pl[L]);
+    k.prm.max_tiles = std::max(k.prm.max_tiles, persist_tiles(k.kind, pl[L].rows, pl[L].ncta));
+  }
+  int fit = 0;
+  if (int e = persist_capacity(k.kind, k.threads, k.prm.max_tiles, fit))
+    return e;
+  if (fit < k.ctas)
+    return ISPM_OK;
+  PersistLane *lanes_d;
+  int *cta_d, *cnt_d;
+  if (int e = mem.put(&lanes_d, sorted.data(), sorted.size()))
+    return e;
+  if (int e = mem.put(&cta_d, cta_lane.data(), cta_lane.size()))
+    return e;
+  if (int e = mem.put(&cnt_d, lane_count.data(), lane_count.size()))
+    return e;
+  PersistParams &P = k.prm;
+  P.lanes = lanes_d;
+  P.cta_lane = cta_d;
+  P.lane_count = cnt_d;
+  P.n_ctas = k.ctas;
+  k.zero_bytes = sizeof(unsigned) * ((size_t)n_lanes + 1);
+  if (int e = mem.get(&k.zero, k.zero_bytes))
+    return e;
+  P.abort = (unsigned *)k.zero;
+  P.bar = P.abort + 1;
+  if (int e = mem.get(&P.part, kPersistParts * (size_t)k.ctas))
+    return e;
+  if (int e = mem.get(&P.out, (size_t)n_lanes))
+    return e;
+  if (cudaMallocHost(&k.host, sizeof(PersistOut) * (size_t)n_lanes) != cudaSuccess ||
+      cudaMallocHost(&k.abort_h, sizeof(unsigned)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(ISPM_ERR_NOMEM, "pinned host allocation");
+  }
+  const int order[] = {R, Batch::P, Q, D, Z, TT};
+  for (int i = 0; i < 6; i++)
+    P.vec[i] = vec[order[i]];
+  P.r64 = r64;
+  P.have_prec = have_prec;
+  P.batch = 1;
+  P.tol = opts.tol;
+  const double ru = inner == ISPM_F32 ? opts.replace_ratio_f32 : opts.replace_ratio_f64;
+  P.ru2 = ru * ru;
+  P.max_iters = opts.max_iters;
+  P.max_refinements = opts.max_refinements;
+  k.on = true;
+  return ISPM_OK;
+}
 
 // Stack the group's lanes into one block-diagonal CSR (identity rows pad
 // every lane to whole tiles) and upload its operators; the FSAI factor of
@@ -829,9 +990,13 @@ int Batch::build_group(Group &g, const int *const *rp, const int *const *ci,
   if ((long long)g.Ain.dev.meta.n_rows != rows || (long long)g.A64.dev.meta.n_rows != rows)
     return fail(ISPM_ERR_INVALID, "stacked operator padded beyond its tiles");
   // lane-segmented launches walk x through registers (the staged shape is
-  // for single systems)
-  g.Ain.lp = register_walk_launch(inner, g.Ain.dev.view());
-  g.A64.lp = register_walk_launch(ISPM_F64, g.A64.dev.view());
+  // for single systems).  How many threads share a row goes by all lanes' rows,
+  // the work of a launch: by the matrix's own rows alone, 41 lanes of 16
+  // systems split each row over up to eight threads, and a 27-point group's
+  // G^T product took 32 us, 11 us since
+  const long long work = (long long)n_tiles * kTile;
+  g.Ain.lp = register_walk_launch(inner, g.Ain.dev.view(), work);
+  g.A64.lp = register_walk_launch(ISPM_F64, g.A64.dev.view(), work);
   if (!have_prec)
     return ISPM_OK;
   std::vector<int> g_rp, g_ci, t_rp, t_ci;
@@ -847,8 +1012,8 @@ int Batch::build_group(Group &g, const int *const *rp, const int *const *ci,
   if (int e = g.Ht.upload(inner, inner, n, t_rp.data(), t_ci.data(), zeros.data(), &g.h_fmt,
                           &pos_t))
     return e;
-  g.G.lp = register_walk_launch(inner, g.G.dev.view());
-  g.Ht.lp = register_walk_launch(inner, g.Ht.dev.view());
+  g.G.lp = register_walk_launch(inner, g.G.dev.view(), work);
+  g.Ht.lp = register_walk_launch(inner, g.Ht.dev.view(), work);
   Mem tmp;
   int *a_rp_d, *a_ci_d, *g_rp_d;
   double *a_v_d, *g_v_d, *gt_v_d;
@@ -983,7 +1148,9 @@ int Batch::build(int n_systems, const int *n_rows, const int *const *rp, const i
   // lane tables
   std::vector<int> tl(n_tiles), lt0(n_lanes), lnt(n_lanes), ab(n_lanes), ac(n_lanes),
       hb_(n_lanes), hc(n_lanes);
-  unsigned cap_a = 1, cap_h = 1;
+  // a lane's partial slots: its tiles' CTAs in tile order, after the earlier
+  // lanes' of all groups (one launch serves several groups)
+  int at_a = 0, at_h = 0;
   for (int L = 0; L < n_lanes; L++) {
     const Lane &ln = lanes[L];
     const Group &g = groups[ln.group];
@@ -991,17 +1158,13 @@ int Batch::build(int n_systems, const int *n_rows, const int *const *rp, const i
       tl[t] = L;
     lt0[L] = ln.tile0;
     lnt[L] = ln.ntile;
-    // a lane's partial slots: its tiles' CTAs, in tile order, after the
-    // group's earlier lanes (a launch covers the group's lane tiles)
-    const unsigned per_a = kTile / g.Ain.cta_rows();
-    ab[L] = (ln.tile0 - g.tile0) * (int)per_a;
-    ac[L] = ln.ntile * (int)per_a;
-    cap_a = std::max(cap_a, (unsigned)g.tiles * per_a);
+    ab[L] = at_a;
+    ac[L] = ln.ntile * (kTile / (int)g.Ain.cta_rows());
+    at_a += ac[L];
     if (have_prec) {
-      const unsigned per_h = kTile / g.Ht.cta_rows();
-      hb_[L] = (ln.tile0 - g.tile0) * (int)per_h;
-      hc[L] = ln.ntile * (int)per_h;
-      cap_h = std::max(cap_h, (unsigned)g.tiles * per_h);
+      hb_[L] = at_h;
+      hc[L] = ln.ntile * (kTile / (int)g.Ht.cta_rows());
+      at_h += hc[L];
     }
   }
   for (const Group &g : groups) {
@@ -1033,9 +1196,9 @@ int Batch::build(int n_systems, const int *n_rows, const int *const *rp, const i
     return e;
   if (int e = mem.get(&ib, 5 * nl))
     return e;
-  if (int e = mem.get(&part_a, cap_a))
+  if (int e = mem.get(&part_a, (size_t)std::max(at_a, 1)))
     return e;
-  if (int e = mem.get(&part_h, cap_h))
+  if (int e = mem.get(&part_h, (size_t)std::max(at_h, 1)))
     return e;
   if (int e = mem.get(&t_pq, nl))
     return e;
@@ -1090,6 +1253,8 @@ int Batch::build(int n_systems, const int *n_rows, const int *const *rp, const i
   ISPM_CUDA_TRY(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
   ISPM_CUDA_TRY(cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming));
   ISPM_CUDA_TRY(cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming));
+  if (int e = init_persist())
+    return e;
   ISPM_CUDA_TRY(cudaDeviceSynchronize());
   return ISPM_OK;
 }

@@ -479,10 +479,12 @@ ispm_launch_params default_launch(int x_dtype, const ispm_slell_view &m)
   return register_walk_launch(x_dtype, m);
 }
 
-ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m)
+ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m,
+                                        long long rows)
 {
   (void)x_dtype;
   ispm_launch_params p{};
+  const double work_rows = rows ? (double)rows : (double)m.n_rows;
   const unsigned esz = m.elm_dtype == ISPM_F64 ? 8 : m.elm_dtype == ISPM_F32 ? 4 : 2;
   const unsigned hmax = m.var_height ? m.min_slice_height : m.slice_height;
   // one 128-bit load of elements per thread and step, at most 4 rows
@@ -495,7 +497,7 @@ ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m)
   // only when rows alone do not.
   const double avg_width = m.n_rows ? (double)m.n_elms / (double)m.n_rows : 1.0;
   const double want_threads = 148.0 * 2048.0;
-  const double row_threads = (double)m.n_rows / H;
+  const double row_threads = work_rows / H;
   unsigned P = 1;
   if (row_threads < want_threads)
     P = pow2_ceil((unsigned)(want_threads / (row_threads > 1 ? row_threads : 1)));

@@ -194,6 +194,13 @@ int Operator::upload(int vec_dtype, int elm_dtype, int n, const int *rp, const i
                  : fail(ISPM_ERR_INVALID, "no sliced-ELL shape accepted the operator");
   fmt = cands[k];
   clear_error();
+  max_diags = 0;
+  if (best.diags && !best.var_height && best.hblock == 1)
+    for (unsigned s = 0; s < best.n_slices; s++) {
+      const unsigned *rec = best.slice_ptr.data() + 3 * (size_t)s;
+      const unsigned wide = (rec[3] - rec[0]) / best.slice_height;
+      max_diags = std::max(max_diags, (int)(wide - (rec[4] - rec[1]) / best.slice_height));
+    }
   if (value_pos)
     if (int st = value_map(best, n, rp, ci, *value_pos))
       return st;

@@ -46,6 +46,7 @@ struct Operator {
   std::shared_ptr<float> diag_mem;
   float *diag = nullptr;
   float inv_scale = 1.f;
+  int max_diags = 0;  // most diagonals of a slice (0 without diagonal blocks)
 
   // Convert (n x n CSR, FP64 values stored as elm_dtype) and upload in the
   // min-bytes shape, or in `force`.  value_pos: CSR entry -> element slot,
@@ -71,9 +72,9 @@ struct Operator {
     }
     return launch_spmv(vdt, lp, dev.view(), x, y, s, skip, ep, pdl);
   }
-  int apply_lanes(int vdt, const void *x, void *y, cudaStream_t s, const SpmvLanes &ln) const
+  LaneOp lane_op(const void *x, void *y, const SpmvLanes &ln) const
   {
-    return launch_spmv_lanes(vdt, lp, dev.view(), x, y, s, ln);
+    return LaneOp{lp, dev.view(), x, y, ln};
   }
   unsigned grid() const { return spmv_grid(lp, dev.view()); }
   unsigned cta_rows() const { return spmv_cta_rows(lp, dev.view()); }

@@ -43,6 +43,7 @@
 #include "nvtx_range.h"
 #include "operator.h"
 #include "pcg_state.h"
+#include "persist.h"
 #include "sblas_impl.h"
 #include "spmv_launch.h"
 
@@ -604,6 +605,17 @@ struct Solver {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   std::vector<double> history;
   int replacements = 0, restarts = 0;
+  // one cooperative launch a solve (persist.cu) for systems that fit L2
+  struct Persist {
+    bool on = false;
+    PersistParams prm;
+    PersistLane lane;
+    PersistKind kind;
+    int ctas = 0, threads = 0;
+    char *dev = nullptr;   // abort flag, count | PersistOut, history | lane, tables
+    char *host = nullptr;  // pinned mirror of the results
+    int history_cap = 0;
+  } pk;
   // ISPM_SOLVER_VERBOSE=1: one stderr line per solver phase (diagnostics)
   bool verbose = getenv("ISPM_SOLVER_VERBOSE") && atoi(getenv("ISPM_SOLVER_VERBOSE")) > 0;
 
@@ -613,6 +625,8 @@ struct Solver {
       cudaGraphExecDestroy(graph);
     if (st_host)
       cudaFreeHost(st_host);
+    if (pk.host)
+      cudaFreeHost(pk.host);
     if (ev_in)
       cudaEventDestroy(ev_in);
     if (ev_out)
@@ -841,8 +855,162 @@ struct Solver {
     return launched("fold correction");
   }
 
+  // Results of a persistent solve: counters (zeroed before the launch), then
+  // what the host reads back.
+  static constexpr size_t kPkZero = 16, kPkHist = 64;  // (abort flag, count; history read back)
+  static constexpr size_t kPkBack = sizeof(PersistOut) + kPkHist * sizeof(double);
+
+  // Decide whether solves run as one cooperative launch, and prepare it.
+  // The line is kPersistMaxBytes of matrices and vectors an iteration.  Whole
+  // solves, this way against the step kernels: 27-point 72^3 mixed 1.65 / 2.83
+  // ms, 20^3 mixed 0.65 / 2.01 ms, 7-point 24^3 FP64 0.51 / 1.00 ms.
+  int init_persist()
+  {
+    Persist &k = pk;
+    PersistLane &l = k.lane;
+    double bytes = (double)Ain.bytes() + 11.0 * esize() * n_pad;
+    if (!persist_op(Ain, 0, l.A) || !persist_op(A64, 0, l.A64) ||
+        Ain.dev.meta.elm_dtype != inner)
+      return ISPM_OK;
+    if (have_prec) {
+      const int ge = G.dev.meta.elm_dtype;
+      if (!persist_op(G, 0, l.G) || !persist_op(Ht, 0, l.Ht) || ge != Ht.dev.meta.elm_dtype ||
+          (ge != inner && !(inner == ISPM_F32 && ge == ISPM_F16)))
+        return ISPM_OK;
+      k.kind.factor_f16 = ge == ISPM_F16;
+      bytes += (double)G.bytes() + (double)Ht.bytes();
+    }
+    if (bytes > kPersistMaxBytes || opts.max_refinements > 100000)
+      return ISPM_OK;
+    l.rows = n_pad;
+    l.n = n;
+    k.kind.inner = inner;
+    k.kind.pipelined = !classic;
+    const int sms = device_sm_count();
+    unsigned low = std::min(Ain.dev.meta.slice_height, A64.dev.meta.slice_height);
+    if (have_prec)
+      low = std::min({low, G.dev.meta.slice_height, Ht.dev.meta.slice_height});
+    k.kind.shape =
+        persist_shape(n_pad, sms * 1024.0, (double)Ain.dev.meta.n_elms / n_pad, low);
+    // one CTA an SM, no more threads than rows give work to: a meeting's sums
+    // and barriers cost by the warp
+    const long long want = (k.kind.shape == kQuarter ? 4LL : 1LL) * n_pad;
+    const long long each = (want + sms - 1) / sms;
+    k.threads = (int)std::min(1024LL, std::max(128LL, (each + 127) / 128 * 128));
+    k.ctas = (int)std::max(1LL, std::min<long long>((want + k.threads - 1) / k.threads, sms));
+    k.prm.max_tiles = persist_tiles(k.kind, n_pad, k.ctas);
+    int most = 0;
+    if (int e = persist_capacity(k.kind, k.threads, k.prm.max_tiles, most))
+      return e;
+    if (most < k.ctas)
+      return ISPM_OK;
+    l.ncta = k.ctas;
+    k.history_cap = std::max(opts.max_refinements, 0) + 8;
+    const size_t hist = std::max<size_t>(kPkHist, (size_t)k.history_cap) * sizeof(double);
+    const size_t tables = sizeof(PersistLane) + sizeof(int) * (size_t)(k.ctas + 1);
+    if (int e = mem.get(&k.dev, kPkZero + sizeof(PersistOut) + hist + tables))
+      return e;
+    if (cudaMallocHost(&k.host, kPkZero + kPkBack) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ISPM_ERR_NOMEM, "pinned host allocation");
+    }
+    PersistParams &P = k.prm;
+    P.n_ctas = k.ctas;
+    if (int e = mem.get(&P.part, kPersistParts * (size_t)k.ctas))
+      return e;
+    P.abort = (unsigned *)k.dev;
+    P.bar = P.abort + 1;
+    P.out = (PersistOut *)(k.dev + kPkZero);
+    P.history = (double *)(k.dev + kPkZero + sizeof(PersistOut));
+    P.history_cap = k.history_cap;
+    char *tab = k.dev + kPkZero + sizeof(PersistOut) + hist;
+    P.lanes = (const PersistLane *)tab;
+    P.lane_count = (const int *)(tab + sizeof(PersistLane));
+    P.cta_lane = P.lane_count + 1;
+    std::vector<int> head((size_t)k.ctas + 1, 0);
+    head[0] = 1;
+    ISPM_CUDA_TRY(cudaMemcpy((void *)P.lane_count, head.data(), head.size() * sizeof(int),
+                             cudaMemcpyHostToDevice));
+    ISPM_CUDA_TRY(cudaMemcpy((void *)P.lanes, &l, sizeof l, cudaMemcpyHostToDevice));
+    const int cl[] = {R, Solver::P, Q, D, Z, TT};
+    const int pl[] = {R, U, W, M, Solver::P, Solver::S, Q, Z, D, TT};
+    if (classic)
+      for (int i = 0; i < 6; i++)
+        P.vec[i] = vec[cl[i]];
+    else
+      for (int i = 0; i < 10; i++)
+        P.vec[i] = vec[pl[i]];
+    P.r64 = r64;
+    P.have_prec = have_prec;
+    P.tol = opts.tol;
+    const double ru = inner == ISPM_F32 ? opts.replace_ratio_f32 : opts.replace_ratio_f64;
+    P.ru2 = ru * ru;
+    P.max_iters = opts.max_iters;
+    P.max_refinements = opts.max_refinements;
+    k.on = true;
+    return ISPM_OK;
+  }
+
+  // (after a value update: the FP16 factor's scale is part of the lane)
+  int refresh_persist()
+  {
+    if (!pk.on)
+      return ISPM_OK;
+    pk.lane.G.inv_scale = G.inv_scale;
+    pk.lane.Ht.inv_scale = Ht.inv_scale;
+    ISPM_CUDA_TRY(cudaMemcpy((void *)pk.prm.lanes, &pk.lane, sizeof pk.lane,
+                             cudaMemcpyHostToDevice));
+    return ISPM_OK;
+  }
+
+  int solve_persistent(const double *b, double *x, ispm_solve_stats *stats, cudaStream_t s)
+  {
+    auto t0 = std::chrono::steady_clock::now();
+    history.clear();
+    Persist &k = pk;
+    k.prm.b = b;
+    k.prm.x = x;
+    ISPM_CUDA_TRY(cudaMemsetAsync(k.dev, 0, kPkZero, s));
+    if (int e = persist_launch(k.prm, k.kind, k.ctas, k.threads, s))
+      return e;
+    ISPM_CUDA_TRY(cudaMemcpyAsync(k.host, k.dev, kPkZero + kPkBack, cudaMemcpyDeviceToHost, s));
+    ISPM_CUDA_TRY(cudaStreamSynchronize(s));
+    if (((const unsigned *)k.host)[0])
+      return fail(ISPM_ERR_TIMEOUT, "persistent solve: a group of CTAs waited too long");
+    const PersistOut &o = *(const PersistOut *)(k.host + kPkZero);
+    const int kept = std::min(o.n_history, k.history_cap);
+    history.resize((size_t)std::max(kept, 0));
+    if (kept > (int)kPkHist)
+      ISPM_CUDA_TRY(cudaMemcpy(history.data(), k.prm.history, sizeof(double) * kept,
+                               cudaMemcpyDeviceToHost));
+    else if (kept > 0)
+      std::memcpy(history.data(), k.host + kPkZero + sizeof(PersistOut), sizeof(double) * kept);
+    replacements = o.replacements;
+    restarts = o.restarts;
+    if (verbose)
+      fprintf(stderr, "[ispm solver] %s one launch: %d iterations, %d phases, true=%.3e\n",
+              inner == ISPM_F32 ? "f32" : "f64", o.iterations, o.n_history, o.rel);
+    ispm_solve_stats out{};
+    out.iterations = o.iterations;
+    out.refinements = o.replacements + o.restarts;
+    out.true_relres = o.rel;
+    out.converged = o.status != ISPM_ERR_INVALID && o.rel <= opts.tol;
+    out.status = o.status;
+    out.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    if (stats)
+      *stats = out;
+    if (o.status == ISPM_ERR_INVALID)
+      return fail(ISPM_ERR_INVALID, "the right-hand side holds a NaN or infinite value");
+    if (o.status != ISPM_OK)
+      return fail(o.status, "solve stopped at relative residual %.3e after %d iterations", o.rel,
+                  o.iterations);
+    return ISPM_OK;
+  }
+
   int solve(const double *b, double *x, ispm_solve_stats *stats, cudaStream_t s)
   {
+    if (pk.on)
+      return solve_persistent(b, x, stats, s);
     auto t0 = std::chrono::steady_clock::now();
     history.clear();
     replacements = restarts = 0;
@@ -1183,7 +1351,7 @@ int update_values(Solver &S, const double *vals, bool on_device)
     cudaGraphExecDestroy(S.graph);
     S.graph = nullptr;
   }
-  return ISPM_OK;
+  return S.refresh_persist();
 }
 
 }  // namespace
@@ -1410,6 +1578,8 @@ int ispm_solver_create(int n, const int *row_ptr, const int *cols, const double 
     if (e)
       return e;
   }
+  if (int e = S.init_persist())
+    return e;
   *out = h.release();
   return ISPM_OK;
 }

@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
+#include <vector>
 
 #include "cuda_util.cuh"
 #include "spmv_launch.h"
@@ -248,7 +249,7 @@ __device__ __forceinline__ void load_window(const T *__restrict__ x, unsigned ba
 }
 
 template <class T, class E, int H, int W, bool VAR, bool DIAG, bool LANES>
-__device__ __forceinline__ void spmv_body(const SpmvArgs<T, E> &a)
+__device__ __forceinline__ void spmv_body(const SpmvArgs<T, E> &a, unsigned bid)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_wait();             // inputs of a programmatic launch are final from here
@@ -259,7 +260,7 @@ __device__ __forceinline__ void spmv_body(const SpmvArgs<T, E> &a)
   const unsigned t = threadIdx.x & (tps - 1);
   const unsigned slice_in_cta = threadIdx.x >> a.log2_tps;
   const unsigned spb = blockDim.x >> a.log2_tps;
-  unsigned cta = blockIdx.x;
+  unsigned cta = bid;
   const T *__restrict__ xp = a.x;
   T *__restrict__ yp = a.y;
   long long shift = 0;
@@ -270,7 +271,7 @@ __device__ __forceinline__ void spmv_body(const SpmvArgs<T, E> &a)
     // names the matrix tile it reads and the lane tile it serves
     static_assert(!VAR, "lane-segmented launches use a fixed slice height");
     const unsigned per = 1024u / (spb * a.slice_height);
-    const unsigned vt = blockIdx.x / per, q = blockIdx.x - vt * per;
+    const unsigned vt = bid / per, q = bid - vt * per;
     const int2 e = __ldg(a.ln.vt + vt);
     lane = __ldg(a.ln.tile_lane + e.y);
     if (__ldg(a.ln.done + lane))
@@ -451,41 +452,48 @@ __device__ __forceinline__ void spmv_body(const SpmvArgs<T, E> &a)
 template <class T, class E, int H, int W, bool VAR, bool DIAG>
 __global__ void __launch_bounds__(1024) slell_spmv_kernel(SpmvArgs<T, E> a)
 {
-  spmv_body<T, E, H, W, VAR, DIAG, false>(a);
+  spmv_body<T, E, H, W, VAR, DIAG, false>(a, blockIdx.x);
 }
 
-// Lane-segmented instances: bounded to two 1024-thread CTAs' registers per
-// SM (the virtual-tile set-up costs registers the single-system instances do
-// not have).
+// Lane-segmented products of up to kMaxLaneOps operators in one launch: CTAs
+// first[k] .. first[k + 1] - 1 serve operator k.  Operators of one kind
+// (rows a thread, hblock width, diagonal blocks, CTA size) share a launch
+// whatever their slice heights, so a batch whose systems fall into several
+// shapes fills the GPU with one launch a product and its iteration stays a
+// chain of programmatic launches.
+template <class T, class E> struct LaneOps {
+  SpmvArgs<T, E> a[kMaxLaneOps];
+  unsigned first[kMaxLaneOps + 1];
+  int n;
+};
+
+// Bounded to two 1024-thread CTAs' registers per SM (the virtual-tile set-up
+// costs registers the single-system instances do not have).
 template <class T, class E, int H, int W, bool DIAG>
-__global__ void __launch_bounds__(1024, 2) slell_spmv_lanes_kernel(SpmvArgs<T, E> a)
+__global__ void __launch_bounds__(1024, 2)
+    slell_spmv_lanes_kernel(const __grid_constant__ LaneOps<T, E> ops)
 {
-  spmv_body<T, E, H, W, false, DIAG, true>(a);
+  int k = 0;
+  while (k + 1 < ops.n && blockIdx.x >= ops.first[k + 1])
+    k++;
+  spmv_body<T, E, H, W, false, DIAG, true>(ops.a[k], blockIdx.x - ops.first[k]);
 }
 
 #include "spmv_staged.cuh"
 
 
-template <class T, class E, int H, int W, bool VAR, bool DIAG, bool LANES = false>
+template <class T, class E, int H, int W, bool VAR, bool DIAG>
 int launch_one(const SpmvArgs<T, E> &args, unsigned tps, cudaStream_t stream)
 {
   // A fused dot ends every CTA with a block reduction, a fence and an
   // arrival on the counter: 1024-thread CTAs do that a quarter as often
   // (the C2 mixed solve measured 58.2 against 59.5 ms, same iterations).
-  const unsigned block = (!LANES && args.ep.out) ? (tps >= 1024 ? tps : 1024)
-                                                 : (tps >= 256 ? tps : 256);
+  const unsigned block = args.ep.out ? (tps >= 1024 ? tps : 1024) : (tps >= 256 ? tps : 256);
   const unsigned spb = block / tps;
-  // lane-segmented: every virtual tile takes 1024 / (spb * S) CTAs
-  const unsigned grid = LANES ? args.ln.n_vt * (1024u / (spb * args.slice_height))
-                              : (args.n_slices + spb - 1) / spb;
+  const unsigned grid = (args.n_slices + spb - 1) / spb;
   const size_t smem = tps > 32 ? (size_t)block * H * sizeof(T) : 0;
-  cudaError_t e;
-  if constexpr (LANES)
-    e = launch_kernel(slell_spmv_lanes_kernel<T, E, H, W, DIAG>, dim3(grid), dim3(block), smem,
-                      stream, args.pdl != 0, args);
-  else
-    e = launch_kernel(slell_spmv_kernel<T, E, H, W, VAR, DIAG>, dim3(grid), dim3(block), smem,
-                      stream, args.pdl != 0, args);
+  cudaError_t e = launch_kernel(slell_spmv_kernel<T, E, H, W, VAR, DIAG>, dim3(grid), dim3(block),
+                                smem, stream, args.pdl != 0, args);
   if (e == cudaSuccess)
     e = cudaPeekAtLastError();
   if (e != cudaSuccess)
@@ -493,27 +501,41 @@ int launch_one(const SpmvArgs<T, E> &args, unsigned tps, cudaStream_t stream)
   return ISPM_OK;
 }
 
+template <class T, int H, int W, bool DIAG>
+int launch_lanes(const LaneOps<T, T> &ops, unsigned block, bool pdl, cudaStream_t stream)
+{
+  size_t smem = 0;
+  for (int k = 0; k < ops.n; k++)
+    if (ops.a[k].tps > 32)
+      smem = (size_t)block * H * sizeof(T);
+  cudaError_t e = launch_kernel(slell_spmv_lanes_kernel<T, T, H, W, DIAG>, dim3(ops.first[ops.n]),
+                                dim3(block), smem, stream, pdl, ops);
+  if (e == cudaSuccess)
+    e = cudaPeekAtLastError();
+  if (e != cudaSuccess)
+    return fail(ISPM_ERR_CUDA, "SpMV launch: %s", cudaGetErrorString(e));
+  return ISPM_OK;
+}
+
+template <class T, int H>
+int launch_lanes_h(const LaneOps<T, T> &ops, unsigned hblock, bool diags, unsigned block, bool pdl,
+                   cudaStream_t s)
+{
+  switch (hblock) {
+  case 1:
+    return diags ? launch_lanes<T, H, 1, true>(ops, block, pdl, s)
+                 : launch_lanes<T, H, 1, false>(ops, block, pdl, s);
+  case 2: return launch_lanes<T, H, 2, false>(ops, block, pdl, s);
+  case 4: return launch_lanes<T, H, 4, false>(ops, block, pdl, s);
+  }
+  return fail(ISPM_ERR_INVALID, "hblock %u", hblock);
+}
+
 template <class T, class E, int H>
 int launch_h(const SpmvArgs<T, E> &args, const ispm_slell_view &m, unsigned tps,
-             cudaStream_t s, bool lanes)
+             cudaStream_t s)
 {
   const bool V = m.var_height != 0, D = m.diags != 0;
-  if (lanes) {
-    if constexpr (std::is_same<T, E>::value) {
-      if (V)
-        return fail(ISPM_ERR_INVALID, "lane-segmented SpMV needs a fixed slice height");
-      switch (m.hblock) {
-      case 1:
-        return D ? launch_one<T, E, H, 1, false, true, true>(args, tps, s)
-                 : launch_one<T, E, H, 1, false, false, true>(args, tps, s);
-      case 2: return launch_one<T, E, H, 2, false, false, true>(args, tps, s);
-      case 4: return launch_one<T, E, H, 4, false, false, true>(args, tps, s);
-      }
-      return fail(ISPM_ERR_INVALID, "hblock %u", m.hblock);
-    } else {
-      return fail(ISPM_ERR_INVALID, "lane-segmented SpMV needs equal vector and element types");
-    }
-  }
   switch (m.hblock) {
   case 1:
     if (V)
@@ -531,33 +553,18 @@ int launch_h(const SpmvArgs<T, E> &args, const ispm_slell_view &m, unsigned tps,
   return fail(ISPM_ERR_INVALID, "hblock %u", m.hblock);
 }
 
+// The arguments every launch of matrix m shares.
 template <class T, class E>
-int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void *x, void *y,
-              cudaStream_t s, const int *skip, const SpmvDot *ep, const SpmvLanes *ln = nullptr,
-              bool pdl = false, const SpmvSplit *split = nullptr)
+int fill_args(SpmvArgs<T, E> &a, const ispm_launch_params &p, const ispm_slell_view &m,
+              const void *x, void *y)
 {
-  SpmvArgs<T, E> a;
-  a.pdl = pdl ? 1 : 0;
+  a.pdl = 0;
   a.dg = nullptr;
   a.inv_scale = 1.f;
   a.st_slots = a.st_slot_bytes = a.st_x_off = 0;
-  if constexpr (std::is_same<E, __half>::value) {
-    if (!split || (split->diag && !aligned(split->diag, 16)))
-      return fail(ISPM_ERR_INVALID,
-                  "FP16 elements need their scale (and a 16-byte aligned split diagonal)");
-    a.dg = split->diag;
-    a.inv_scale = split->inv_scale;
-  }
-  a.skip = skip;
-  a.ep = ep ? *ep : SpmvDot{};
-  a.ln = ln ? *ln : SpmvLanes{};
-  if (ep && ep->out) {
-    const unsigned block = p.N >= 256 ? p.N : 256;
-    const unsigned grid = (m.n_slices + block / p.N - 1) / (block / p.N);
-    if (grid > ep->part_capacity)
-      return fail(ISPM_ERR_INVALID, "fused dot needs %u partial slots, has %u", grid,
-                  ep->part_capacity);
-  }
+  a.skip = nullptr;
+  a.ep = SpmvDot{};
+  a.ln = SpmvLanes{};
   a.sp = m.slice_ptr;
   a.cols = m.cols;
   a.elms = static_cast<const E *>(m.elms);
@@ -573,20 +580,50 @@ int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void 
   if (!aligned(m.elms, p.H * sizeof(E)) || !aligned(m.cols, p.H * sizeof(unsigned)) ||
       !aligned(y, p.H * sizeof(T)))
     return fail(ISPM_ERR_INVALID, "matrix arrays or y not aligned to H=%u elements", p.H);
+  return ISPM_OK;
+}
+
+template <class T, class E>
+int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void *x, void *y,
+              cudaStream_t s, const int *skip, const SpmvDot *ep, bool pdl = false,
+              const SpmvSplit *split = nullptr)
+{
+  if constexpr (std::is_same<E, __half>::value)
+    if (!split || (split->diag && !aligned(split->diag, 16)))
+      return fail(ISPM_ERR_INVALID,
+                  "FP16 elements need their scale (and a 16-byte aligned split diagonal)");
+  SpmvArgs<T, E> a;
+  const int bad = fill_args(a, p, m, x, y);
+  a.pdl = pdl ? 1 : 0;
+  if constexpr (std::is_same<E, __half>::value) {
+    a.dg = split->diag;
+    a.inv_scale = split->inv_scale;
+  }
+  a.skip = skip;
+  a.ep = ep ? *ep : SpmvDot{};
+  if (ep && ep->out) {
+    const unsigned block = p.N >= 256 ? p.N : 256;
+    const unsigned grid = (m.n_slices + block / p.N - 1) / (block / p.N);
+    if (grid > ep->part_capacity)
+      return fail(ISPM_ERR_INVALID, "fused dot needs %u partial slots, has %u", grid,
+                  ep->part_capacity);
+  }
+  if (bad)
+    return bad;
   if constexpr (std::is_same<T, float>::value) {
     StageInfo si;
-    if (!ln && staged_shape(ISPM_F32, p, m, x, si, a.st_slots, a.st_slot_bytes, a.st_x_off))
+    if (staged_shape(ISPM_F32, p, m, x, si, a.st_slots, a.st_slot_bytes, a.st_x_off))
       return launch_staged<E>(a, si, s);
   }
   switch (p.H) {
-  case 1: return launch_h<T, E, 1>(a, m, p.N, s, ln != nullptr);
-  case 2: return launch_h<T, E, 2>(a, m, p.N, s, ln != nullptr);
-  case 4: return launch_h<T, E, 4>(a, m, p.N, s, ln != nullptr);
+  case 1: return launch_h<T, E, 1>(a, m, p.N, s);
+  case 2: return launch_h<T, E, 2>(a, m, p.N, s);
+  case 4: return launch_h<T, E, 4>(a, m, p.N, s);
   case 8:
     // eight rows a thread: FP32 vectors, one column per stored index
     if constexpr (std::is_same<T, float>::value) {
-      if (ln || m.hblock != 1)
-        return fail(ISPM_ERR_INVALID, "H = 8 needs hblock 1 and a single system");
+      if (m.hblock != 1)
+        return fail(ISPM_ERR_INVALID, "H = 8 needs hblock 1");
       const bool V = m.var_height != 0, D = m.diags != 0;
       if (V)
         return D ? launch_one<T, E, 8, 1, true, true>(a, p.N, s)
@@ -652,27 +689,78 @@ unsigned spmv_cta_rows(const ispm_launch_params &p, const ispm_slell_view &m)
   return block / p.N * m.slice_height;
 }
 
-int launch_spmv_lanes(int x_dtype, const ispm_launch_params &p, const ispm_slell_view &m,
-                      const void *x, void *y, cudaStream_t s, const SpmvLanes &lanes)
+static int check_lane_op(int x_dtype, const LaneOp &op)
 {
-  int st = check_launch(x_dtype, p, m);
+  const ispm_slell_view &m = op.m;
+  int st = check_launch(x_dtype, op.p, m);
   if (st)
     return st;
-  if (m.n_slices == 0)
-    return ISPM_OK;
-  if (!x || !y || !m.slice_ptr || (m.n_elms && (!m.elms)) || (m.n_cols_arr && !m.cols) ||
+  const SpmvLanes &lanes = op.ln;
+  if (!op.x || !op.y || !m.slice_ptr || (m.n_elms && (!m.elms)) || (m.n_cols_arr && !m.cols) ||
       !lanes.tile_lane || !lanes.done || !lanes.vt)
     return fail(ISPM_ERR_INVALID, "NULL pointer");
   if (lanes.out && (!lanes.v || !lanes.part || !lanes.ticket || !lanes.cta_beg ||
                     !lanes.cta_cnt || !lanes.lane_tile0))
     return fail(ISPM_ERR_INVALID, "lane dot without its buffers");
-  if (m.var_height || 1024u % spmv_cta_rows(p, m) != 0)
+  if (m.var_height || 1024u % spmv_cta_rows(op.p, m) != 0)
     return fail(ISPM_ERR_INVALID, "a CTA of this launch does not fit one 1024-row tile");
   if (x_dtype != m.elm_dtype)
     return fail(ISPM_ERR_INVALID, "lane-segmented SpMV needs equal vector and element types");
-  if (x_dtype == ISPM_F32)
-    return launch_te<float, float>(p, m, x, y, s, nullptr, nullptr, &lanes);
-  return launch_te<double, double>(p, m, x, y, s, nullptr, nullptr, &lanes);
+  if (op.p.H > 4)
+    return fail(ISPM_ERR_INVALID, "H = %u in a lane-segmented SpMV", op.p.H);
+  return ISPM_OK;
+}
+
+template <class T>
+static int launch_lane_ops(int x_dtype, const LaneOp *ops, int n, cudaStream_t s, bool pdl,
+                           int *launches)
+{
+  auto block_of = [](const LaneOp &o) { return o.p.N >= 256 ? o.p.N : 256u; };
+  std::vector<char> done((size_t)n, 0);
+  for (int i = 0; i < n; i++) {
+    if (done[i] || ops[i].m.n_slices == 0)
+      continue;
+    LaneOps<T, T> k;
+    k.n = 0;
+    k.first[0] = 0;
+    const unsigned block = block_of(ops[i]);
+    for (int j = i; j < n && k.n < kMaxLaneOps; j++) {
+      const LaneOp &o = ops[j];
+      if (done[j] || o.m.n_slices == 0 || o.p.H != ops[i].p.H || o.m.hblock != ops[i].m.hblock ||
+          (o.m.diags != 0) != (ops[i].m.diags != 0) || block_of(o) != block)
+        continue;
+      if (int e = check_lane_op(x_dtype, o))
+        return e;
+      if (int e = fill_args(k.a[k.n], o.p, o.m, o.x, o.y))
+        return e;
+      k.a[k.n].ln = o.ln;
+      // every virtual tile takes 1024 / (rows a CTA) CTAs
+      k.first[k.n + 1] = k.first[k.n] + o.ln.n_vt * (1024u / spmv_cta_rows(o.p, o.m));
+      k.n++;
+      done[j] = 1;
+    }
+    if (!k.first[k.n])
+      continue;
+    int e = ISPM_OK;
+    const bool d = ops[i].m.diags != 0;
+    switch (ops[i].p.H) {
+    case 1: e = launch_lanes_h<T, 1>(k, ops[i].m.hblock, d, block, pdl, s); break;
+    case 2: e = launch_lanes_h<T, 2>(k, ops[i].m.hblock, d, block, pdl, s); break;
+    default: e = launch_lanes_h<T, 4>(k, ops[i].m.hblock, d, block, pdl, s); break;
+    }
+    if (e)
+      return e;
+    if (launches)
+      ++*launches;
+  }
+  return ISPM_OK;
+}
+
+int launch_spmv_lanes(int x_dtype, const LaneOp *ops, int n, cudaStream_t s, bool pdl,
+                      int *launches)
+{
+  return x_dtype == ISPM_F32 ? launch_lane_ops<float>(x_dtype, ops, n, s, pdl, launches)
+                             : launch_lane_ops<double>(x_dtype, ops, n, s, pdl, launches);
 }
 
 unsigned spmv_grid(const ispm_launch_params &p, const ispm_slell_view &m)
@@ -702,14 +790,14 @@ int launch_spmv(int x_dtype, const ispm_launch_params &p, const ispm_slell_view 
   if (!x || !y || !m.slice_ptr || (m.n_elms && (!m.elms)) || (m.n_cols_arr && !m.cols))
     return fail(ISPM_ERR_INVALID, "NULL pointer");
   if (x_dtype == ISPM_F32 && m.elm_dtype == ISPM_BF16)
-    return launch_te<float, __nv_bfloat16>(p, m, x, y, s, skip, ep, nullptr, pdl);
+    return launch_te<float, __nv_bfloat16>(p, m, x, y, s, skip, ep, pdl);
   if (x_dtype == ISPM_F32 && m.elm_dtype == ISPM_F16)
-    return launch_te<float, __half>(p, m, x, y, s, skip, ep, nullptr, pdl, split);
+    return launch_te<float, __half>(p, m, x, y, s, skip, ep, pdl, split);
   if (x_dtype == ISPM_F32)
-    return launch_te<float, float>(p, m, x, y, s, skip, ep, nullptr, pdl);
+    return launch_te<float, float>(p, m, x, y, s, skip, ep, pdl);
   if (m.elm_dtype == ISPM_F32)
-    return launch_te<double, float>(p, m, x, y, s, skip, ep, nullptr, pdl);
-  return launch_te<double, double>(p, m, x, y, s, skip, ep, nullptr, pdl);
+    return launch_te<double, float>(p, m, x, y, s, skip, ep, pdl);
+  return launch_te<double, double>(p, m, x, y, s, skip, ep, pdl);
 }
 
 }  // namespace ispm

@@ -83,9 +83,21 @@ int launch_spmv(int x_dtype, const ispm_launch_params &p, const ispm_slell_view 
                 const void *x, void *y, cudaStream_t s, const int *skip = nullptr,
                 const SpmvDot *ep = nullptr, bool pdl = false,
                 const SpmvSplit *split = nullptr);
-// Lane-segmented launch (fixed slice height, T == E only; grid: n_vt tiles).
-int launch_spmv_lanes(int x_dtype, const ispm_launch_params &p, const ispm_slell_view &m,
-                      const void *x, void *y, cudaStream_t s, const SpmvLanes &lanes);
+// Lane-segmented products (fixed slice height, T == E, H <= 4; grid: n_vt
+// tiles each): operators of one kind share a launch, up to kMaxLaneOps of
+// them.  They must not depend on one another.  pdl: launch as programmatic
+// dependents of the stream's previous kernel.  *launches (may be NULL) grows
+// by the launches made.
+constexpr int kMaxLaneOps = 8;
+struct LaneOp {
+  ispm_launch_params p;
+  ispm_slell_view m;
+  const void *x;
+  void *y;
+  SpmvLanes ln;
+};
+int launch_spmv_lanes(int x_dtype, const LaneOp *ops, int n, cudaStream_t s, bool pdl,
+                      int *launches);
 // CTAs a launch of matrix m with params p uses (partials a fused dot needs).
 unsigned spmv_grid(const ispm_launch_params &p, const ispm_slell_view &m);
 // Rows one CTA of such a launch covers (fixed slice height).
@@ -167,8 +179,10 @@ struct DeviceSlell {
 ispm_launch_params default_launch(int x_dtype, const ispm_slell_view &m);
 // The same heuristic restricted to the register walk (several rows per
 // thread, x gathered through the read-only path): the shapes the
-// lane-segmented launches take.
-ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m);
+// lane-segmented launches take.  rows: the rows a launch works on where that
+// is more than the matrix's own (several lanes sharing it), else 0.
+ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m,
+                                        long long rows = 0);
 
 // d.elms[map[k]] = vals[k] for k < n (device arrays; vals FP32 or FP64).
 // Same from the slot side: d.elms[s] = vals[inv[s]] for every element slot
