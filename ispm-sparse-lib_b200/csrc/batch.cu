@@ -912,8 +912,14 @@ int Batch::init_persist()
     return fail(ISPM_ERR_NOMEM, "pinned host allocation");
   }
   const int order[] = {R, Batch::P, Q, D, Z, TT};
-  for (int i = 0; i < 6; i++)
-    P.vec[i] = vec[order[i]];
+  for (int i = 0; i < 8; i++) {
+    if (i < 6) {
+      P.vec[i] = vec[order[i]];
+    } else if (int e = inner == ISPM_F32 ? mem.get((float **)&P.vec[i], (size_t)n_stack)
+                                         : mem.get((double **)&P.vec[i], (size_t)n_stack)) {
+      return e;
+    }
+  }
   P.r64 = r64;
   P.have_prec = have_prec;
   P.batch = 1;

@@ -932,10 +932,10 @@ struct Solver {
     ISPM_CUDA_TRY(cudaMemcpy((void *)P.lane_count, head.data(), head.size() * sizeof(int),
                              cudaMemcpyHostToDevice));
     ISPM_CUDA_TRY(cudaMemcpy((void *)P.lanes, &l, sizeof l, cudaMemcpyHostToDevice));
-    const int cl[] = {R, Solver::P, Q, D, Z, TT};
+    const int cl[] = {R, Solver::P, Q, D, Z, TT, U, W};
     const int pl[] = {R, U, W, M, Solver::P, Solver::S, Q, Z, D, TT};
     if (classic)
-      for (int i = 0; i < 6; i++)
+      for (int i = 0; i < 8; i++)
         P.vec[i] = vec[cl[i]];
     else
       for (int i = 0; i < 10; i++)

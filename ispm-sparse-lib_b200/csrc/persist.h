@@ -58,8 +58,8 @@ struct PersistParams {
   const PersistLane *lanes = nullptr;  // device; lanes of one group in a row
   const int *cta_lane = nullptr;       // CTA -> first lane of its group
   const int *lane_count = nullptr;     // lanes of that group, by first lane
-  // inner vectors.  Classic: R, P, Q, D, Z, T; pipelined: R, U, W, M, P, S, Q,
-  // Z, D, T
+  // inner vectors.  Classic: R, P, Q, D, Z, T and second ones of R and P;
+  // pipelined: R, U, W, M, P, S, Q, Z, D, T
   void *vec[10] = {};
   double *r64 = nullptr;
   const double *b = nullptr;
