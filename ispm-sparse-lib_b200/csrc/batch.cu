@@ -866,6 +866,7 @@ int Batch::init_persist()
     return ISPM_OK;
   int most = 0;
   k.kind.inner = inner;
+  k.kind.wide = false;  // (1.81 against 2.43 ms: 32 warps an SM over several small groups)
   k.kind.shape = persist_shape((double)n_stack, (double)device_sm_count() * 1024, 4.0, low);
   if (int e = persist_capacity(k.kind, k.threads, 1, most))
     return e;

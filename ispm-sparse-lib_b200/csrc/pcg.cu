@@ -890,13 +890,15 @@ struct Solver {
     unsigned low = std::min(Ain.dev.meta.slice_height, A64.dev.meta.slice_height);
     if (have_prec)
       low = std::min({low, G.dev.meta.slice_height, Ht.dev.meta.slice_height});
-    k.kind.shape =
-        persist_shape(n_pad, sms * 1024.0, (double)Ain.dev.meta.n_elms / n_pad, low);
+    const int wide = kPersistWideThreads;
+    k.kind.shape = persist_shape(n_pad, (double)sms * wide,
+                                 (double)Ain.dev.meta.n_elms / n_pad, low);
     // one CTA an SM, no more threads than rows give work to: a meeting's sums
     // and barriers cost by the warp
-    const long long want = (k.kind.shape == kQuarter ? 4LL : 1LL) * n_pad;
+    const int per = k.kind.shape == kRow4 ? 4 : k.kind.shape == kRow2 ? 2 : 1;
+    const long long want = (k.kind.shape == kQuarter ? 4LL * n_pad : (long long)n_pad / per);
     const long long each = (want + sms - 1) / sms;
-    k.threads = (int)std::min(1024LL, std::max(128LL, (each + 127) / 128 * 128));
+    k.threads = (int)std::min<long long>(wide, std::max(128LL, (each + 63) / 64 * 64));
     k.ctas = (int)std::max(1LL, std::min<long long>((want + k.threads - 1) / k.threads, sms));
     k.prm.max_tiles = persist_tiles(k.kind, n_pad, k.ctas);
     int most = 0;

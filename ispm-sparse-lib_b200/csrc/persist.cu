@@ -167,7 +167,7 @@ struct Tile {
 };
 
 // One group's view of itself and the sums its CTAs agree on.
-template <int V, int LP> struct Group {
+template <int V, int LP, bool WIDE> struct Group {
   const PersistParams &P;
   const PersistLane &L;  // in shared memory
   double *sh;            // shared: kSums x 32 warp sums, then as many of the readers
@@ -411,7 +411,7 @@ template <int V, int LP> struct Group {
   __device__ __forceinline__ void spmv(const PersistOp &op, int which, const X x, Pre pre, F f)
   {
     constexpr int rpw = kTileRows;         // rows a warp takes at once
-    constexpr int U = V == 1 ? 8 : 8 / V;  // entries a block
+    constexpr int U = (WIDE ? 16 : 8) / V;  // entries a block
     constexpr unsigned np = 1u << LP;
     const unsigned *cols = op.cols;
     const E *elms = static_cast<const E *>(op.elms);
@@ -986,8 +986,10 @@ __device__ __forceinline__ void solve_pipelined(G &g, int slot)
   });
 }
 
-template <class T, class E, bool PIPE, int V, int LP>
-__global__ void __launch_bounds__(1024, 1) persist_kernel(const __grid_constant__ PersistParams P)
+// WIDE: at most 640 threads a CTA (96 registers each) with sixteen entries'
+// loads of a row in flight; else 1024 threads with eight.
+template <class T, class E, bool PIPE, int V, int LP, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kPersistWideThreads : 1024, 1) persist_kernel(const __grid_constant__ PersistParams P)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double sh[2 * kSums * 32];
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(1024, 1) persist_kernel(const __grid_constant_
       reinterpret_cast<unsigned *>(&lane)[w] =
           reinterpret_cast<const unsigned *>(P.lanes + first + k)[w];
     __syncthreads();
-    Group<V, LP> g(P, lane, sh, ok, reinterpret_cast<Tile *>(smem_raw));
+    Group<V, LP, WIDE> g(P, lane, sh, ok, reinterpret_cast<Tile *>(smem_raw));
     g.start(first + k);
     if constexpr (PIPE)
       solve_pipelined<T, E>(g, first + k);
@@ -1015,26 +1017,30 @@ __global__ void __launch_bounds__(1024, 1) persist_kernel(const __grid_constant_
 
 using Kernel = void (*)(PersistParams);
 
-template <class T, class E, bool PIPE> Kernel pick_shape(PersistShape w)
+template <class T, class E, bool PIPE, bool WIDE> Kernel pick_shape(PersistShape w)
 {
   switch (w) {
-  case kRow4: return persist_kernel<T, E, PIPE, 4, 0>;
-  case kRow2: return persist_kernel<T, E, PIPE, 2, 0>;
-  case kRow1: return persist_kernel<T, E, PIPE, 1, 0>;
-  default: return persist_kernel<T, E, PIPE, 1, 2>;
+  case kRow4: return persist_kernel<T, E, PIPE, 4, 0, WIDE>;
+  case kRow2: return persist_kernel<T, E, PIPE, 2, 0, WIDE>;
+  case kRow1: return persist_kernel<T, E, PIPE, 1, 0, WIDE>;
+  default: return persist_kernel<T, E, PIPE, 1, 2, WIDE>;
   }
 }
 
 // (FP32 pipelined solves stay on the step kernels: no default takes them)
 Kernel pick(const PersistKind &k)
 {
+  if (!k.wide)  // batches
+    return k.pipelined || k.factor_f16 ? nullptr
+           : k.inner == ISPM_F64       ? pick_shape<double, double, false, false>(k.shape)
+                                       : pick_shape<float, float, false, false>(k.shape);
   if (k.inner == ISPM_F64)
-    return k.pipelined ? pick_shape<double, double, true>(k.shape)
-                       : pick_shape<double, double, false>(k.shape);
+    return k.pipelined ? pick_shape<double, double, true, true>(k.shape)
+                       : pick_shape<double, double, false, true>(k.shape);
   if (k.pipelined)
     return nullptr;
-  return k.factor_f16 ? pick_shape<float, __half, false>(k.shape)
-                      : pick_shape<float, float, false>(k.shape);
+  return k.factor_f16 ? pick_shape<float, __half, false, true>(k.shape)
+                      : pick_shape<float, float, false, true>(k.shape);
 }
 
 }  // namespace
@@ -1089,11 +1095,11 @@ int persist_capacity(const PersistKind &k, int threads, int max_tiles, int &ctas
 
 PersistShape persist_shape(double rows, double threads, double width, unsigned min_height)
 {
-  if (rows >= 2 * threads && min_height >= 128)
+  if (rows > 2 * threads && min_height >= 128)
     return kRow4;
-  if (rows >= threads && min_height >= 64)
+  if (rows > threads && min_height >= 64)
     return kRow2;
-  return 16 * rows <= threads && width >= 4 ? kQuarter : kRow1;
+  return 10 * rows <= threads && width >= 4 ? kQuarter : kRow1;
 }
 
 int persist_launch(const PersistParams &p, const PersistKind &k, int ctas, int threads,

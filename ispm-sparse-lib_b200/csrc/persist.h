@@ -36,8 +36,9 @@ struct PersistLane {
 
 // Rows a thread of the walk (4, 2, 1), or four threads a row.
 enum PersistShape { kRow4, kRow2, kRow1, kQuarter };
-// The shape for `rows` rows of about `width` entries on `threads` threads;
-// min_height: the shortest slice height of the operators.
+// The shape for `rows` rows of about `width` entries on `threads` threads, the
+// fewest rows a thread that leave each thread one turn; min_height: the
+// shortest slice height of the operators.
 PersistShape persist_shape(double rows, double threads, double width, unsigned min_height);
 
 struct PersistKind {
@@ -45,7 +46,12 @@ struct PersistKind {
   bool pipelined = false;  // (FP64 only)
   bool factor_f16 = false; // FP16 factor values (FP32 vectors)
   PersistShape shape = kRow1;
+  // sixteen entries' loads of a thread in flight, at most kPersistWideThreads
+  // threads a CTA (against eight and 1024: 27-point mixed solves 0.98 / 1.11 ms
+  // at 56^3, 1.50 / 1.64 ms at 72^3)
+  bool wide = true;
 };
+constexpr int kPersistWideThreads = 640;
 
 // What a lane's solve reports.
 struct PersistOut {
