@@ -866,8 +866,14 @@ int Batch::init_persist()
     return ISPM_OK;
   int most = 0;
   k.kind.inner = inner;
-  k.kind.wide = false;  // (1.81 against 2.43 ms: 32 warps an SM over several small groups)
-  k.kind.shape = persist_shape((double)n_stack, (double)device_sm_count() * 1024, 4.0, low);
+  // up to three turns of the wide kernel's rows: two wide CTAs an SM, past it
+  // four narrow ones (us, wide / narrow: 117,760 rows in 6 lanes 825 / 1601,
+  // 163,840 in 12 1016 / 1143, 748,544 in 41 2100 / 1907)
+  const double sms = device_sm_count();
+  k.kind.wide = (double)n_stack <= 3.0 * sms * kPersistWideThreads;
+  k.threads = k.kind.wide ? kPersistWideThreads / 2 : 256;
+  k.kind.shape = persist_shape((double)n_stack, sms * (k.kind.wide ? kPersistWideThreads : 1024),
+                               4.0, low);
   if (int e = persist_capacity(k.kind, k.threads, 1, most))
     return e;
   if (most < 1)
