@@ -188,6 +188,7 @@ template <class T>
 __global__ void scalars_kernel(T *alpha, T *beta, const T *gamma, const T *gammaold,
                                const T *delta)
 {
+  pdl_wait();
   // sblas.cu:156-165
   T g = *gamma;
   T b = g / *gammaold;
@@ -223,6 +224,7 @@ __device__ __forceinline__ void ppcg_elem(T a, T b, T nv, T mv, T &p, T &s, T &q
 template <class T>
 __global__ void __launch_bounds__(kThreads) ppcg_vectors_kernel(PpcgVecArgs<T> g)
 {
+  pdl_wait();
   const T a = *g.alpha, b = *g.beta;
   Acc<3> acc{{0.0, 0.0, 0.0}};
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -261,6 +263,7 @@ __global__ void __launch_bounds__(kThreads) ppcg_vectors_kernel(PpcgVecArgs<T> g
   for (long long i = done + i0; i < g.n_elts; i += stride)
     ppcg_elem<T>(a, b, g.n[i], g.m[i], g.p[i], g.s[i], g.q[i], g.z[i], g.x[i], g.r[i], g.u[i],
                  g.w[i], acc);
+  pdl_trigger();
   Acc<3> tot;
   if (finish_grid<3>(acc, g.part, g.ticket, tot) && threadIdx.x == 0) {
     *g.resnorm = (T)tot.v[0];
@@ -306,8 +309,13 @@ template <class T> int ppcg_vectors_launch(PpcgVecArgs<T> g, cudaStream_t st)
           aligned(g.q, 16) && aligned(g.z, 16) && aligned(g.x, 16) && aligned(g.r, 16) &&
           aligned(g.u, 16) && aligned(g.w, 16);
   const int grid = sblas_grid(g.n_elts, g.vec ? 16 / (int)sizeof(T) : 1);
-  ppcg_vectors_kernel<T><<<grid, kThreads, 0, st>>>(g);
-  cudaError_t e = cudaPeekAtLastError();
+  // (a programmatic dependent: launched while the stream's previous kernel,
+  // often the one-thread scalars, ends; it touches nothing before that
+  // kernel's results are final.  Scalars and vectors of 2,000,003 FP32
+  // elements: 31.4 against 35.3 us)
+  cudaError_t e = launch_kernel(ppcg_vectors_kernel<T>, dim3(grid), dim3(kThreads), 0, st, true, g);
+  if (e == cudaSuccess)
+    e = cudaPeekAtLastError();
   if (e != cudaSuccess)
     return fail(ISPM_ERR_CUDA, "ppcg_update_vectors launch: %s", cudaGetErrorString(e));
   return ISPM_OK;
@@ -411,14 +419,17 @@ int ispm_sblas_ppcg_update_scalars(int dtype, void *alpha, void *beta, const voi
     return st;
   if (!alpha || !beta || !gamma || !gammaold || !delta)
     return fail(ISPM_ERR_INVALID, "NULL scalar");
+  cudaError_t e;
   if (dtype == ISPM_F32)
-    scalars_kernel<float><<<1, 1, 0, (cudaStream_t)stream>>>(
-        (float *)alpha, (float *)beta, (const float *)gamma, (const float *)gammaold,
-        (const float *)delta);
+    e = launch_kernel(scalars_kernel<float>, dim3(1), dim3(1), 0, (cudaStream_t)stream, true,
+                      (float *)alpha, (float *)beta, (const float *)gamma,
+                      (const float *)gammaold, (const float *)delta);
   else
-    scalars_kernel<double><<<1, 1, 0, (cudaStream_t)stream>>>(
-        (double *)alpha, (double *)beta, (const double *)gamma, (const double *)gammaold,
-        (const double *)delta);
+    e = launch_kernel(scalars_kernel<double>, dim3(1), dim3(1), 0, (cudaStream_t)stream, true,
+                      (double *)alpha, (double *)beta, (const double *)gamma,
+                      (const double *)gammaold, (const double *)delta);
+  if (e != cudaSuccess)
+    return fail(ISPM_ERR_CUDA, "ppcg_update_scalars launch: %s", cudaGetErrorString(e));
   return launch_status("ppcg_update_scalars");
 }
 
