@@ -341,11 +341,13 @@ template <class E, class V>
 __global__ void refresh_gather_kernel(E *__restrict__ elms, const int *__restrict__ inv,
                                       const V *__restrict__ vals, long long n)
 {
+  pdl_wait();
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
     const int src = __ldcs(inv + k);
     elms[k] = src >= 0 ? (E)__ldg(vals + src) : E(0);
   }
+  pdl_trigger();
 }
 
 int refresh_values_gather(DeviceSlell &d, const int *inv, const void *vals, int val_dtype,
@@ -360,19 +362,18 @@ int refresh_values_gather(DeviceSlell &d, const int *inv, const void *vals, int 
   const bool e32 = d.meta.elm_dtype == ISPM_F32, v32 = val_dtype == ISPM_F32;
   if (d.meta.elm_dtype != ISPM_F32 && d.meta.elm_dtype != ISPM_F64)
     return fail(ISPM_ERR_INVALID, "slot-order refresh of an element type %d", d.meta.elm_dtype);
-  if (e32 && v32)
-    refresh_gather_kernel<float, float><<<blocks, threads, 0, s>>>((float *)d.elms, inv,
-                                                                   (const float *)vals, n);
-  else if (e32)
-    refresh_gather_kernel<float, double><<<blocks, threads, 0, s>>>((float *)d.elms, inv,
-                                                                    (const double *)vals, n);
-  else if (v32)
-    refresh_gather_kernel<double, float><<<blocks, threads, 0, s>>>((double *)d.elms, inv,
-                                                                    (const float *)vals, n);
-  else
-    refresh_gather_kernel<double, double><<<blocks, threads, 0, s>>>((double *)d.elms, inv,
-                                                                     (const double *)vals, n);
-  cudaError_t e = cudaPeekAtLastError();
+  auto run = [&](auto kernel, auto *elms, auto *values) {
+    return launch_kernel(kernel, dim3((unsigned)blocks), dim3(threads), 0, s, true, elms, inv,
+                         values, n);
+  };
+  const float *vf = (const float *)vals;
+  const double *vd = (const double *)vals;
+  cudaError_t e = e32 ? (v32 ? run(refresh_gather_kernel<float, float>, (float *)d.elms, vf)
+                             : run(refresh_gather_kernel<float, double>, (float *)d.elms, vd))
+                      : (v32 ? run(refresh_gather_kernel<double, float>, (double *)d.elms, vf)
+                             : run(refresh_gather_kernel<double, double>, (double *)d.elms, vd));
+  if (e == cudaSuccess)
+    e = cudaPeekAtLastError();
   return e == cudaSuccess ? ISPM_OK
                           : fail(ISPM_ERR_CUDA, "value refresh: %s", cudaGetErrorString(e));
 }

@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
       }
   };
   const long long first = ((long long)blockIdx.x * (kFwdThreads / 32) + w) * 32;
+  pdl_wait();
   load_rows(first);
   load_weights(s, prm);
   __syncthreads();
@@ -283,6 +284,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
           Y[r] = make_float2(y[m][q][0], y[m][q][1]);
       }
   }
+  pdl_trigger();
 }
 
 // One warp's 16 rows of a training step: forward, loss, backward up to the
@@ -492,6 +494,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
   const long long first = (long long)blockIdx.x * kBlockRows;
   const long long step = (long long)gridDim.x * kBlockRows;
+  pdl_wait();
   stage_rows(s.x[0], X, first, M, al16);
   load_weights(s.w, prm);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, w = threadIdx.x >> 5;
@@ -535,6 +538,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       mma(acc1[1], a, b[2], b[3]);
     }
   }
+  pdl_trigger();
   float *out = part + (size_t)blockIdx.x * kPart;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
@@ -612,6 +616,7 @@ __global__ void mlp_adam_kernel(float *__restrict__ prm, float *__restrict__ m,
                                 float *__restrict__ v, const float *__restrict__ grad, float lr,
                                 float b1, float b2, float eps, float c1, float c2, float wd)
 {
+  pdl_wait();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kParams)
     return;
@@ -768,6 +773,7 @@ __global__ void __launch_bounds__(2 * kFeatRows, 4)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FeatSmem &s = *reinterpret_cast<FeatSmem *>(smem_raw);
   constexpr int kT = 2 * kFeatRows;
+  pdl_wait();
   const int tid = threadIdx.x, r0 = blockIdx.x * kFeatRows, rows = min(kFeatRows, n - r0);
   const int first = __ldg(rp + r0), count = __ldg(rp + r0 + rows) - first;
   const bool staged = count <= kFeatCap;
@@ -796,6 +802,7 @@ __global__ void __launch_bounds__(2 * kFeatRows, 4)
     feature_row<I>(i, len, h, s.ci + (e0 - first), s.v + (e0 - first), nx, ny, f);
   else
     feature_row<I>(i, len, h, ci + e0, v + e0, nx, ny, f);
+  pdl_trigger();
   __syncthreads();
   uint32_t *o = reinterpret_cast<uint32_t *>(out + (size_t)r0 * kFeat);
   for (int k = tid; k < rows * (kFeat / 2); k += kT)
@@ -907,8 +914,9 @@ int ispm_mlp_forward(const ispm_mlp *m, long long n_rows, const void *feat_bf16,
     return fail(ISPM_ERR_INVALID, "features must be 4-byte, outputs 8-byte aligned");
   if (n_rows == 0)
     return ISPM_OK;
-  mlp_forward_kernel<<<fwd_grid(n_rows), kFwdThreads, 0, (cudaStream_t)stream>>>(
-      m->prm, (const bf16 *)feat_bf16, (float2 *)out, n_rows);
+  ISPM_CUDA_TRY(launch_kernel(mlp_forward_kernel, dim3(fwd_grid(n_rows)), dim3(kFwdThreads), 0,
+                              (cudaStream_t)stream, true, (const float *)m->prm,
+                              (const bf16 *)feat_bf16, (float2 *)out, n_rows));
   ISPM_CUDA_TRY(cudaPeekAtLastError());
   return ISPM_OK;
 }
@@ -936,9 +944,12 @@ int ispm_mlp_loss_grad(ispm_mlp *m, long long n_rows, const void *feat_bf16,
     m->part_cta = grid;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  mlp_train_kernel<<<grid, kThreads, sizeof(TrainSmem), s>>>(
-      m->prm, (const bf16 *)feat_bf16, (const float2 *)target, (const float2 *)weight, n_rows,
-      1.0f / (float)n_rows, aligned(feat_bf16, 16), m->part);
+  // (programmatic launches: each kernel is set up while the one before it ends
+  // and waits on the device for its results)
+  ISPM_CUDA_TRY(launch_kernel(mlp_train_kernel, dim3(grid), dim3(kThreads), sizeof(TrainSmem), s,
+                              true, (const float *)m->prm, (const bf16 *)feat_bf16,
+                              (const float2 *)target, (const float2 *)weight, n_rows,
+                              1.0f / (float)n_rows, (int)aligned(feat_bf16, 16), m->part));
   ISPM_CUDA_TRY(cudaPeekAtLastError());
   ISPM_CUDA_TRY(launch_kernel(mlp_reduce_kernel, dim3((kPart + 31) / 32), dim3(32 * kReduceWarps), 0,
                               s, true, (const float *)m->part, grid, m->grad));
@@ -966,8 +977,10 @@ int ispm_mlp_adam_step(ispm_mlp *m, float lr, float beta1, float beta2, float ep
   m->step++;
   const float c1 = 1.f - std::pow(beta1, (float)m->step);
   const float c2 = 1.f - std::pow(beta2, (float)m->step);
-  mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-      m->prm, m->m, m->v, m->grad, lr, beta1, beta2, eps, c1, c2, weight_decay);
+  ISPM_CUDA_TRY(launch_kernel(mlp_adam_kernel, dim3((kParams + 255) / 256), dim3(256), 0,
+                              (cudaStream_t)stream, true, m->prm, m->m, m->v,
+                              (const float *)m->grad, lr, beta1, beta2, eps, c1, c2,
+                              weight_decay));
   ISPM_CUDA_TRY(cudaPeekAtLastError());
   return ISPM_OK;
 }
@@ -989,8 +1002,9 @@ int ispm_row_features(int n, const int *row_ptr, const int *cols, const double *
     return e;
   const auto kernel = (long long)nx * ny < (1LL << 29) ? row_features_kernel<int>
                                                        : row_features_kernel<long long>;
-  kernel<<<(n + kFeatRows - 1) / kFeatRows, 2 * kFeatRows, sizeof(FeatSmem),
-           (cudaStream_t)stream>>>(n, row_ptr, cols, vals, nx, ny, (bf16 *)out_bf16);
+  ISPM_CUDA_TRY(launch_kernel(kernel, dim3((n + kFeatRows - 1) / kFeatRows), dim3(2 * kFeatRows),
+                              sizeof(FeatSmem), (cudaStream_t)stream, true, n, row_ptr, cols, vals,
+                              nx, ny, (bf16 *)out_bf16));
   ISPM_CUDA_TRY(cudaPeekAtLastError());
   return ISPM_OK;
 }

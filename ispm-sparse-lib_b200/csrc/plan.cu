@@ -235,7 +235,8 @@ int ispm_plan_execute(ispm_plan *p, const void *x, void *y, void *stream)
     return fail(ISPM_ERR_INVALID, "NULL plan");
   if (!p->dev)
     return fail(ISPM_ERR_INVALID, "plan has no device matrix (SPMV_PLAN_NO_DEVICE)");
-  return launch_spmv(p->vec_dtype, p->params, p->dev->d.view(), x, y, (cudaStream_t)stream);
+  return launch_spmv(p->vec_dtype, p->params, p->dev->d.view(), x, y, (cudaStream_t)stream, nullptr,
+                     nullptr, true);
 }
 
 int ispm_plan_upload(ispm_plan *p)

@@ -612,8 +612,10 @@ int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void 
     return bad;
   if constexpr (std::is_same<T, float>::value) {
     StageInfo si;
-    if (staged_shape(ISPM_F32, p, m, x, si, a.st_slots, a.st_slot_bytes, a.st_x_off))
+    if (staged_shape(ISPM_F32, p, m, x, si, a.st_slots, a.st_slot_bytes, a.st_x_off)) {
+      a.pdl = 0;  // it fetches elements before it waits for the kernel before it
       return launch_staged<E>(a, si, s);
+    }
   }
   switch (p.H) {
   case 1: return launch_h<T, E, 1>(a, m, p.N, s);
@@ -815,7 +817,9 @@ int ispm_launch_spmv(int x_dtype, const ispm_launch_params *p, const ispm_slell_
   ispm::clear_error();
   if (!p || !m)
     return ispm::fail(ISPM_ERR_INVALID, "NULL params or matrix");
-  return ispm::launch_spmv(x_dtype, *p, *m, x, y, (cudaStream_t)stream);
+  // (a programmatic dependent: launched while the stream's previous kernel
+  // ends, it reads nothing before that kernel's results are final)
+  return ispm::launch_spmv(x_dtype, *p, *m, x, y, (cudaStream_t)stream, nullptr, nullptr, true);
 }
 
 int ispm_launch_spmv_split(const ispm_launch_params *p, const ispm_slell_view *m,
@@ -829,7 +833,7 @@ int ispm_launch_spmv_split(const ispm_launch_params *p, const ispm_slell_view *m
     return ispm::fail(ISPM_ERR_INVALID, "the split product takes FP16 elements");
   ispm::SpmvSplit sp{diag, inv_scale};
   return ispm::launch_spmv(ISPM_F32, *p, *m, x, y, (cudaStream_t)stream, nullptr, nullptr,
-                           false, &sp);
+                           true, &sp);
 }
 
 int ispm_spmv_stage_fault(int *code)
