@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "cuda_util.cuh"
+#include "host_pool.h"
 #include "operator.h"
 #include "spmv_launch.h"
 
@@ -337,54 +338,258 @@ __global__ void refresh_bf16_kernel(__nv_bfloat16 *__restrict__ elms,
     elms[__ldcs(map + k)] = __float2bfloat16_rn((float)__ldcs(vals + k));
 }
 
-template <class E, class V>
-__global__ void refresh_gather_kernel(E *__restrict__ elms, const int *__restrict__ inv,
-                                      const V *__restrict__ vals, long long n)
+template <class E> __device__ __forceinline__ E element(double v, double)
 {
+  return (E)v;
+}
+template <> __device__ __forceinline__ __nv_bfloat16 element<__nv_bfloat16>(double v, double)
+{
+  return __float2bfloat16_rn((float)v);
+}
+template <> __device__ __forceinline__ __half element<__half>(double v, double scale)
+{
+  return __double2half(v * scale);
+}
+
+// The power of two that maps *amax into [2^13, 2^14) (1 for 0).
+__device__ __forceinline__ double f16_scale(const double *amax)
+{
+  const double m = amax ? *amax : 0.0;
+  return m > 0.0 ? scalbn(1.0, isfinite(m) ? 13 - ilogb(m) : 14) : 1.0;
+}
+
+// Values through shared memory (SlotMap).  Bound by HBM: 8 bytes of value, 2
+// of map and the element a slot.  61 x 75 x 83 27-point FP64 (10.0 M entries):
+// 43 us (4.2 TB/s); gathering each slot's value from the CSR, 4 bytes of map a
+// slot, took 49 us.
+template <class E, class E2, class V>
+__global__ void __launch_bounds__(256)
+    refresh_chunks_kernel(E *__restrict__ elms, E2 *__restrict__ second,
+                          const int4 *__restrict__ chunk, const unsigned short *__restrict__ idx,
+                          const V *__restrict__ vals, const double *amax)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V *sm = reinterpret_cast<V *>(smem_raw);
   pdl_wait();
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int src = __ldcs(inv + k);
-    elms[k] = src >= 0 ? (E)__ldg(vals + src) : E(0);
+  const int4 c = __ldg(chunk + blockIdx.x);
+  const V *v = vals + c.z;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < c.w; i += 256)
+    sm[i] = __ldcs(v + i);
+  const double scale = f16_scale(amax);
+  __syncthreads();
+  auto value = [&](unsigned k) { return k == 0xffffu ? 0.0 : (double)sm[k]; };
+  if (((c.x | c.y) & 3) == 0) {  // four slots a thread
+    struct __align__(sizeof(E) * 4) Q {
+      E v[4];
+    };
+    struct __align__(sizeof(E2) * 4) Q2 {
+      E2 v[4];
+    };
+#pragma unroll 2
+    for (int i = 4 * threadIdx.x; i < c.y; i += 1024) {
+      const ushort4 k = __ldcs(reinterpret_cast<const ushort4 *>(idx + c.x + i));
+      const double a = value(k.x), b = value(k.y), d = value(k.z), e = value(k.w);
+      *reinterpret_cast<Q *>(elms + c.x + i) =
+          Q{{element<E>(a, scale), element<E>(b, scale), element<E>(d, scale),
+             element<E>(e, scale)}};
+      if (second)
+        *reinterpret_cast<Q2 *>(second + c.x + i) =
+            Q2{{element<E2>(a, scale), element<E2>(b, scale), element<E2>(d, scale),
+                element<E2>(e, scale)}};
+    }
+  } else {
+    for (int i = threadIdx.x; i < c.y; i += 256) {
+      const double a = value(idx[c.x + i]);
+      elms[c.x + i] = element<E>(a, scale);
+      if (second)
+        second[c.x + i] = element<E2>(a, scale);
+    }
   }
   pdl_trigger();
 }
 
-int refresh_values_gather(DeviceSlell &d, const int *inv, const void *vals, int val_dtype,
-                          cudaStream_t s)
+template <class E, class E2, class V>
+__global__ void refresh_gather_kernel(E *__restrict__ elms, E2 *__restrict__ second,
+                                      const int *__restrict__ inv, const V *__restrict__ vals,
+                                      long long n, const double *amax)
 {
-  const long long n = d.meta.n_elms;
-  if (!n)
-    return ISPM_OK;
-  const int threads = 256;
-  const long long blocks =
-      std::min<long long>((n + threads - 1) / threads, (long long)device_sm_count() * 16);
-  const bool e32 = d.meta.elm_dtype == ISPM_F32, v32 = val_dtype == ISPM_F32;
-  if (d.meta.elm_dtype != ISPM_F32 && d.meta.elm_dtype != ISPM_F64)
-    return fail(ISPM_ERR_INVALID, "slot-order refresh of an element type %d", d.meta.elm_dtype);
-  auto run = [&](auto kernel, auto *elms, auto *values) {
-    return launch_kernel(kernel, dim3((unsigned)blocks), dim3(threads), 0, s, true, elms, inv,
-                         values, n);
+  pdl_wait();
+  const double scale = f16_scale(amax);
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const int src = __ldcs(inv + k);
+    const double v = src >= 0 ? (double)__ldg(vals + src) : 0.0;
+    elms[k] = element<E>(v, scale);
+    if (second)
+      second[k] = element<E2>(v, scale);
+  }
+  pdl_trigger();
+}
+
+std::vector<unsigned> slice_begins(const HostSlell &h)
+{
+  const unsigned spe = 1 + (h.hblock > 1) + (h.var_height ? 1 : 0) + (h.diags ? 2 : 0);
+  std::vector<unsigned> b(h.n_slices + 1, 0u);
+  for (unsigned s = 0; s <= h.n_slices && h.n_slices; s++)
+    b[s] = h.slice_ptr[(size_t)spe * s];
+  return b;
+}
+
+void SlotMap::release()
+{
+  for (void *p : {(void *)chunk, (void *)idx, (void *)inv})
+    if (p)
+      cudaFree(p);
+  chunk = nullptr;
+  idx = nullptr;
+  inv = nullptr;
+  n_chunks = max_entries = 0;
+  n_slots = 0;
+}
+
+int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<unsigned> &pos)
+{
+  // a chunk: slices up to 3,072 entries (24 KB of FP64 values, eight CTAs an
+  // SM), a taller slice alone up to 8,192
+  constexpr int kFull = 3072, kMost = 8192;
+  release();
+  n_slots = slice_begin.back();
+  std::vector<int> in((size_t)n_slots, -1);
+  parallel_for((long long)pos.size(), [&](long long a, long long b) {
+    for (long long k = a; k < b; k++)
+      in[pos[(size_t)k]] = (int)k;
+  });
+  const long long n_sl = (long long)slice_begin.size() - 1;
+  std::vector<int2> span((size_t)n_sl);  // first and last entry of a slice
+  parallel_for(n_sl, [&](long long a, long long b) {
+    for (long long s = a; s < b; s++) {
+      int l = 0x7fffffff, h = -1;
+      for (unsigned p = slice_begin[s]; p < slice_begin[s + 1]; p++)
+        if (in[p] >= 0) {
+          l = std::min(l, in[p]);
+          h = std::max(h, in[p]);
+        }
+      span[(size_t)s] = make_int2(l, h);
+    }
+  });
+  std::vector<int4> ch;
+  bool runs = true;
+  int lo = 0, hi = -1, most = 0;  // the open chunk's entries
+  unsigned first = 0;
+  auto close = [&](unsigned end) {
+    if (end > first) {
+      const int n = hi >= lo ? hi - lo + 1 : 0;
+      ch.push_back(make_int4((int)first, (int)(end - first), n ? lo : 0, n));
+      most = std::max(most, n);
+    }
+    first = end;
+    lo = 0;
+    hi = -1;
   };
-  const float *vf = (const float *)vals;
-  const double *vd = (const double *)vals;
-  cudaError_t e = e32 ? (v32 ? run(refresh_gather_kernel<float, float>, (float *)d.elms, vf)
-                             : run(refresh_gather_kernel<float, double>, (float *)d.elms, vd))
-                      : (v32 ? run(refresh_gather_kernel<double, float>, (double *)d.elms, vf)
-                             : run(refresh_gather_kernel<double, double>, (double *)d.elms, vd));
+  for (size_t s = 0; s < (size_t)n_sl && runs; s++) {
+    const int l = span[s].x, h = span[s].y;
+    runs = h < l || h - l < kMost;
+    if (h < l)
+      continue;  // (padding alone joins the open chunk)
+    if (hi >= lo && std::max(hi, h) - std::min(lo, l) >= kFull)
+      close(slice_begin[s]);
+    lo = hi >= lo ? std::min(lo, l) : l;
+    hi = std::max(hi, h);
+  }
+  if (runs)
+    close(slice_begin.back());
+  if (runs && !ch.empty()) {
+    std::vector<unsigned short> ix((size_t)n_slots, 0xffffu);
+    parallel_for((long long)ch.size(), [&](long long a, long long b) {
+      for (long long q = a; q < b; q++) {
+        const int4 c = ch[(size_t)q];
+        for (int i = 0; i < c.y; i++)
+          if (in[(size_t)c.x + i] >= 0)
+            ix[(size_t)c.x + i] = (unsigned short)(in[(size_t)c.x + i] - c.z);
+      }
+    });
+    ISPM_CUDA_TRY(cudaMalloc(&chunk, ch.size() * sizeof(int4)));
+    ISPM_CUDA_TRY(cudaMemcpy(chunk, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    ISPM_CUDA_TRY(cudaMalloc(&idx, ix.size() * sizeof(unsigned short)));
+    ISPM_CUDA_TRY(
+        cudaMemcpy(idx, ix.data(), ix.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+    n_chunks = (int)ch.size();
+    max_entries = most;
+    return ISPM_OK;
+  }
+  ISPM_CUDA_TRY(cudaMalloc(&inv, std::max<size_t>(in.size(), 1) * sizeof(int)));
+  if (!in.empty())
+    ISPM_CUDA_TRY(cudaMemcpy(inv, in.data(), in.size() * sizeof(int), cudaMemcpyHostToDevice));
+  return ISPM_OK;
+}
+
+namespace {
+
+template <class E, class E2, class V>
+int refresh_slots_t(E *elms, E2 *second, const SlotMap &m, const V *vals, const double *amax,
+                    cudaStream_t s)
+{
+  cudaError_t e;
+  if (m.chunk) {
+    const size_t smem = (size_t)m.max_entries * sizeof(V);
+    const auto kernel = refresh_chunks_kernel<E, E2, V>;
+    e = smem > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)smem)
+                         : cudaSuccess;
+    if (e == cudaSuccess)
+      e = launch_kernel(kernel, dim3(m.n_chunks), dim3(256), smem, s, true, elms, second,
+                        (const int4 *)m.chunk, (const unsigned short *)m.idx, vals, amax);
+  } else {
+    const long long blocks =
+        std::min<long long>((m.n_slots + 255) / 256, (long long)device_sm_count() * 16);
+    e = launch_kernel(refresh_gather_kernel<E, E2, V>, dim3((unsigned)blocks), dim3(256), 0, s, true,
+                      elms, second, (const int *)m.inv, vals, m.n_slots, amax);
+  }
   if (e == cudaSuccess)
     e = cudaPeekAtLastError();
   return e == cudaSuccess ? ISPM_OK
                           : fail(ISPM_ERR_CUDA, "value refresh: %s", cudaGetErrorString(e));
 }
 
-// elms[map[k]] = FP16(vals[k] * scale), rounded to nearest.
-__global__ void refresh_f16_kernel(__half *__restrict__ elms, const unsigned *__restrict__ map,
-                                   const double *__restrict__ vals, long long n, double scale)
+template <class V>
+int refresh_slots_v(DeviceSlell &d, const SlotMap &m, const V *vals, const double *amax,
+                    cudaStream_t s)
 {
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x)
-    elms[__ldcs(map + k)] = __double2half(__ldcs(vals + k) * scale);
+  switch (d.meta.elm_dtype) {
+  case ISPM_F32: return refresh_slots_t((float *)d.elms, (float *)nullptr, m, vals, amax, s);
+  case ISPM_F64: return refresh_slots_t((double *)d.elms, (double *)nullptr, m, vals, amax, s);
+  case ISPM_BF16:
+    return refresh_slots_t((__nv_bfloat16 *)d.elms, (__nv_bfloat16 *)nullptr, m, vals, amax, s);
+  }
+  return refresh_slots_t((__half *)d.elms, (__half *)nullptr, m, vals, amax, s);
+}
+
+}  // namespace
+
+int refresh_slots(DeviceSlell &d, const SlotMap &map, const void *vals, int val_dtype,
+                  cudaStream_t s, DeviceSlell *second, const double *amax)
+{
+  if (map.n_slots != d.meta.n_elms || (second && second->meta.n_elms != d.meta.n_elms))
+    return fail(ISPM_ERR_INVALID, "a slot map of %lld slots for %lld elements", map.n_slots,
+                d.meta.n_elms);
+  if ((d.meta.elm_dtype == ISPM_F16) != (amax != nullptr))
+    return fail(ISPM_ERR_INVALID, "FP16 elements (alone) are refreshed with their scale");
+  if (!map.n_slots)
+    return ISPM_OK;
+  if (second) {  // an FP64 matrix and its FP32 or FP64 copy
+    if (d.meta.elm_dtype != ISPM_F64 || val_dtype != ISPM_F64 ||
+        (second->meta.elm_dtype != ISPM_F32 && second->meta.elm_dtype != ISPM_F64))
+      return fail(ISPM_ERR_INVALID, "a joint refresh of element types %d and %d",
+                  d.meta.elm_dtype, second->meta.elm_dtype);
+    return second->meta.elm_dtype == ISPM_F32
+               ? refresh_slots_t((double *)d.elms, (float *)second->elms, map,
+                                 (const double *)vals, amax, s)
+               : refresh_slots_t((double *)d.elms, (double *)second->elms, map,
+                                 (const double *)vals, amax, s);
+  }
+  return val_dtype == ISPM_F32 ? refresh_slots_v(d, map, (const float *)vals, amax, s)
+                               : refresh_slots_v(d, map, (const double *)vals, amax, s);
 }
 
 // *out = max |v_k| as the bit pattern of a non-negative double (which orders
@@ -392,50 +597,25 @@ __global__ void refresh_f16_kernel(__half *__restrict__ elms, const unsigned *__
 __global__ void absmax_kernel(const double *__restrict__ v, long long n, unsigned long long *out)
 {
   double m = 0.0;
+#pragma unroll 4
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x)
-    m = fmax(m, fabs(v[k]));
+    m = fmax(m, fabs(__ldg(v + k)));
   for (int off = 16; off > 0; off >>= 1)
     m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
   if ((threadIdx.x & 31) == 0)
     atomicMax(out, (unsigned long long)__double_as_longlong(m));
 }
 
-int device_absmax(const double *vals, long long n, double &out)
+int absmax_async(const double *vals, long long n, double *out, cudaStream_t s)
 {
-  out = 0.0;
-  if (!n)
-    return ISPM_OK;
-  unsigned long long *d = nullptr;
-  ISPM_CUDA_TRY(cudaMalloc(&d, sizeof(unsigned long long)));
-  unsigned long long h = 0;
-  cudaError_t e = cudaMemset(d, 0, sizeof(h));
-  if (e == cudaSuccess) {
-    const long long blocks = std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8);
-    absmax_kernel<<<blocks, 256>>>(vals, n, d);
-    e = cudaPeekAtLastError();
-  }
-  if (e == cudaSuccess)
-    e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
-  cudaFree(d);
-  if (e != cudaSuccess)
-    return fail(ISPM_ERR_CUDA, "absolute maximum: %s", cudaGetErrorString(e));
-  std::memcpy(&out, &h, sizeof(out));
-  return ISPM_OK;
-}
-
-int refresh_values_f16(DeviceSlell &d, const unsigned *map, const double *vals, long long n,
-                       double scale, cudaStream_t s)
-{
-  if (d.meta.elm_dtype != ISPM_F16)
-    return fail(ISPM_ERR_INVALID, "scaled FP16 refresh of an element type %d", d.meta.elm_dtype);
+  ISPM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double), s));
   if (!n)
     return ISPM_OK;
   const long long blocks = std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8);
-  refresh_f16_kernel<<<blocks, 256, 0, s>>>((__half *)d.elms, map, vals, n, scale);
-  cudaError_t e = cudaPeekAtLastError();
-  return e == cudaSuccess ? ISPM_OK
-                          : fail(ISPM_ERR_CUDA, "value refresh: %s", cudaGetErrorString(e));
+  absmax_kernel<<<blocks, 256, 0, s>>>(vals, n, (unsigned long long *)out);
+  ISPM_CUDA_TRY(cudaPeekAtLastError());
+  return ISPM_OK;
 }
 
 int refresh_values(DeviceSlell &d, const unsigned *map, const void *vals, int val_dtype,

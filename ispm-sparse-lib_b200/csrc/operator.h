@@ -54,11 +54,12 @@ struct Operator {
   // bf16_values: keep the FP32 elements as BF16 on the device.
   // f16_values: FP16 element storage for values written later on the device
   // (set_f16_values); the uploaded values must be exact binary16 values
-  // (the solver passes zeros).
+  // (the solver passes zeros).  begins: slice_begins of the converted matrix.
   int upload(int vec_dtype, int elm_dtype, int n, const int *rp, const int *ci,
              const double *v, const ispm_slell_params *force = nullptr,
              std::vector<unsigned> *value_pos = nullptr, bool fixed_height = false,
-             bool bf16_values = false, bool f16_values = false);
+             bool bf16_values = false, bool f16_values = false,
+             std::vector<unsigned> *begins = nullptr);
   // Upload the FP16 split of an n x n FP64 CSR (split_f16): the off-diagonal
   // entries in the min-bytes sliced-ELL shape with FP16 elements, the
   // corrected diagonal as an FP32 vector.  FP32 vectors only.

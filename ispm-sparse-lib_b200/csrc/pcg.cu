@@ -572,19 +572,21 @@ struct Solver {
   // reordered solves: perm[new] = old, and b / x in the solver's order
   int *perm = nullptr;
   double *b_perm = nullptr, *x_perm = nullptr;
-  // opts.refresh: what ispm_solver_update_values needs.  pos_*: CSR entry
-  // (solver order) -> element slot of each device copy of A; entry_src: for
+  // opts.refresh: what ispm_solver_update_values needs.  map_a64: where the
+  // slots of the FP64 A take their values (solver order), and those of the
+  // inner A where it has the same shape; else map_ain; entry_src: for
   // a renumbered solve, solver-order entry -> caller-order entry; a_v: A's
   // values in solver order (device); fsai: the factor build's device arrays.
   bool refreshable = false;
   long long nnz_a = 0;
-  unsigned *pos_ain = nullptr, *pos_a64 = nullptr;
+  SlotMap map_a64, map_ain;
   int *entry_src = nullptr;
   double *a_v = nullptr, *a_raw = nullptr;
   struct FsaiArrays {
     int *a_rp = nullptr, *a_ci = nullptr, *g_rp = nullptr;
-    unsigned *t_of = nullptr, *pos_g = nullptr, *pos_t = nullptr, *fb = nullptr;
-    double *g_v = nullptr, *gt_v = nullptr;
+    unsigned *fb = nullptr;
+    double *g_v = nullptr, *amax = nullptr;
+    std::shared_ptr<SlotMap> map_g, map_t;  // G's and G^T's slots from G's entries
     long long nnz_g = 0;
     int max_pattern = 0;
     bool f16 = false;
@@ -1179,14 +1181,6 @@ struct ispm_solver {
 namespace ispm {
 namespace {
 
-__global__ void scatter_kernel(double *__restrict__ out, const unsigned *__restrict__ at,
-                               const double *__restrict__ in, long long n)
-{
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (long long)gridDim.x * blockDim.x)
-    out[at[k]] = in[k];
-}
-
 template <class T> int to_device(DevMem &mem, T **d, const T *h, size_t count)
 {
   if (int e = mem.get(d, count))
@@ -1197,39 +1191,37 @@ template <class T> int to_device(DevMem &mem, T **d, const T *h, size_t count)
 }
 
 // FSAI values of G from A's device values a_v (solver order, the pattern of
-// f.a_rp / f.a_ci), G^T's by the scatter, both written into the device
-// factor matrices through their CSR-entry -> slot maps (legacy stream).
+// f.a_rp / f.a_ci), written into both device factor matrices (legacy stream).
 int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
 {
   if (int e = fsai_build_values(S.n, f.max_pattern, f.a_rp, f.a_ci, a_v, f.g_rp, f.g_v, f.fb, 0))
     return e;
-  const int blocks = grid_for(f.nnz_g);
-  scatter_kernel<<<blocks, kThreads>>>(f.gt_v, f.t_of, f.g_v, f.nnz_g);
-  ISPM_CUDA_TRY(cudaPeekAtLastError());
-  if (f.f16) {
-    // one power-of-two scale for both factors: the largest magnitude lands
-    // in [2^13, 2^14), below the binary16 maximum (65504)
-    double amax = 0.0;
-    if (int e = device_absmax(f.g_v, f.nnz_g, amax))
+  // FP16: one power-of-two scale for both factors, formed on the device: the
+  // largest magnitude lands in [2^13, 2^14), below the binary16 maximum (65504)
+  const double *amax_d = f.f16 ? f.amax : nullptr;
+  if (f.f16)
+    if (int e = absmax_async(f.g_v, f.nnz_g, f.amax, 0))
       return e;
+  if (int e = refresh_slots(S.G.dev, *f.map_g, f.g_v, ISPM_F64, 0, nullptr, amax_d))
+    return e;
+  if (int e = refresh_slots(S.Ht.dev, *f.map_t, f.g_v, ISPM_F64, 0, nullptr, amax_d))
+    return e;
+  struct {
+    double amax;
+    unsigned fb[2];
+  } back;
+  // (the count sits behind the maximum)
+  ISPM_CUDA_TRY(cudaMemcpy(&back, f.amax, sizeof back, cudaMemcpyDeviceToHost));
+  S.fsai_fallbacks = back.fb[0];
+  if (f.f16) {
     int ex = 0;
-    if (amax > 0.0)
-      std::frexp(amax, &ex);
-    const double sc = std::ldexp(1.0, amax > 0.0 ? 14 - ex : 0);
+    if (back.amax > 0.0)
+      std::frexp(back.amax, &ex);
+    const double sc = std::ldexp(1.0, back.amax > 0.0 ? 14 - ex : 0);
     if (!(sc > 0.0) || !std::isfinite(sc) || sc > 0x1p126 || sc < 0x1p-126)
       return fail(ISPM_ERR_INVALID, "FP16 factor: magnitudes out of the FP32 scale range");
-    if (int e = refresh_values_f16(S.G.dev, f.pos_g, f.g_v, f.nnz_g, sc, 0))
-      return e;
-    if (int e = refresh_values_f16(S.Ht.dev, f.pos_t, f.gt_v, f.nnz_g, sc, 0))
-      return e;
     S.G.inv_scale = S.Ht.inv_scale = (float)(1.0 / sc);
-  } else {
-    if (int e = refresh_values(S.G.dev, f.pos_g, f.g_v, ISPM_F64, f.nnz_g, 0))
-      return e;
-    if (int e = refresh_values(S.Ht.dev, f.pos_t, f.gt_v, ISPM_F64, f.nnz_g, 0))
-      return e;
   }
-  ISPM_CUDA_TRY(cudaMemcpy(&S.fsai_fallbacks, f.fb, sizeof(unsigned), cudaMemcpyDeviceToHost));
   return ISPM_OK;
 }
 
@@ -1241,7 +1233,7 @@ int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
 int build_fsai_on_device(Solver &S, int n, const int *rp, const int *ci, const double *v)
 {
   std::vector<int> g_rp, g_ci, t_rp, t_ci;
-  std::vector<unsigned> t_of, pos_g, pos_t;
+  std::vector<unsigned> t_of, pos_g, pos_t, begin_g, begin_t;
   if (int e = fsai_lower_pattern(n, rp, ci, g_rp, g_ci))
     return e;
   fsai_transpose_pattern(n, g_rp, g_ci, t_rp, t_ci, t_of);
@@ -1250,10 +1242,10 @@ int build_fsai_on_device(Solver &S, int n, const int *rp, const int *ci, const d
   const bool f16 = S.inner == ISPM_F32 && S.opts.factor_f16;
   const bool bf16 = S.inner == ISPM_F32 && S.opts.factor_bf16 && !f16;
   if (int e = S.G.upload(S.inner, S.inner, n, g_rp.data(), g_ci.data(), zeros.data(), nullptr,
-                         &pos_g, false, bf16, f16))
+                         &pos_g, false, bf16, f16, &begin_g))
     return e;
   if (int e = S.Ht.upload(S.inner, S.inner, n, t_rp.data(), t_ci.data(), zeros.data(), nullptr,
-                          &pos_t, false, bf16, f16))
+                          &pos_t, false, bf16, f16, &begin_t))
     return e;
   if (f16) {
     // FP16 factor values in diagonal blocks with at least eight stored
@@ -1291,18 +1283,19 @@ int build_fsai_on_device(Solver &S, int n, const int *rp, const int *ci, const d
   }
   if (int e = to_device(mem, &f.g_rp, g_rp.data(), g_rp.size()))
     return e;
-  if (int e = to_device(mem, &f.t_of, t_of.data(), nnz_g))
+  for (size_t k = 0; k < nnz_g; k++)  // G's entry -> slot of G^T
+    t_of[k] = pos_t[t_of[k]];
+  f.map_g = std::make_shared<SlotMap>();
+  f.map_t = std::make_shared<SlotMap>();
+  if (int e = f.map_g->build(begin_g, pos_g))
     return e;
-  if (int e = to_device(mem, &f.pos_g, pos_g.data(), nnz_g))
-    return e;
-  if (int e = to_device(mem, &f.pos_t, pos_t.data(), nnz_g))
+  if (int e = f.map_t->build(begin_t, t_of))
     return e;
   if (int e = mem.get(&f.g_v, nnz_g))
     return e;
-  if (int e = mem.get(&f.gt_v, nnz_g))
+  if (int e = mem.get(&f.amax, 2))
     return e;
-  if (int e = mem.get(&f.fb, 1))
-    return e;
+  f.fb = (unsigned *)(f.amax + 1);
   if (int e = fsai_values(S, f, a_v_d))
     return e;
   if (S.refreshable) {
@@ -1339,10 +1332,12 @@ int update_values(Solver &S, const double *vals, bool on_device)
     ISPM_CUDA_TRY(cudaPeekAtLastError());
     a_v = S.a_v;
   }
-  if (int e = refresh_values(S.A64.dev, S.pos_a64, a_v, ISPM_F64, nnz, 0))
+  const bool joint = S.map_ain.empty();
+  if (int e = refresh_slots(S.A64.dev, S.map_a64, a_v, ISPM_F64, 0, joint ? &S.Ain.dev : nullptr))
     return e;
-  if (int e = refresh_values(S.Ain.dev, S.pos_ain, a_v, ISPM_F64, nnz, 0))
-    return e;
+  if (!joint)
+    if (int e = refresh_slots(S.Ain.dev, S.map_ain, a_v, ISPM_F64, 0))
+      return e;
   if (S.fsai_kept)
     if (int e = fsai_values(S, S.fsai, a_v))
       return e;
@@ -1484,14 +1479,14 @@ int ispm_solver_create(int n, const int *row_ptr, const int *cols, const double 
     return fail(ISPM_ERR_NOMEM, "host allocation while reordering");
   }
   try {
-    std::vector<unsigned> pos_ain, pos_a64;
+    std::vector<unsigned> pos_ain, pos_a64, begin_ain, begin_a64;
     std::vector<unsigned> *want_ain = S.refreshable ? &pos_ain : nullptr;
     std::vector<unsigned> *want_a64 = S.refreshable ? &pos_a64 : nullptr;
     if (S.inner == ISPM_F32 && S.opts.matrix_f16) {
       if (int e = S.Ain.upload_split_f16(n, row_ptr, cols, vals))
         return e;
-    } else if (int e = S.Ain.upload(S.inner, S.inner, n, row_ptr, cols, vals, nullptr,
-                                    want_ain)) {
+    } else if (int e = S.Ain.upload(S.inner, S.inner, n, row_ptr, cols, vals, nullptr, want_ain,
+                                    false, false, false, &begin_ain)) {
       return e;
     }
     // the FP64 operator of the reliable updates takes the inner matrix's
@@ -1499,14 +1494,16 @@ int ispm_solver_create(int n, const int *row_ptr, const int *cols, const double 
     // for the off-diagonal part alone): then A64 gets its own min-bytes shape
     const bool split = S.inner == ISPM_F32 && S.opts.matrix_f16;
     if (int e = S.A64.upload(ISPM_F64, ISPM_F64, n, row_ptr, cols, vals,
-                             split ? nullptr : &S.Ain.fmt, want_a64))
+                             split ? nullptr : &S.Ain.fmt, want_a64, false, false, false,
+                             &begin_a64))
       return e;
     if (S.refreshable) {
       const size_t nnz = (size_t)S.nnz_a;
-      if (int e = to_device(S.mem, &S.pos_ain, pos_ain.data(), nnz))
+      if (int e = S.map_a64.build(begin_a64, pos_a64))
         return e;
-      if (int e = to_device(S.mem, &S.pos_a64, pos_a64.data(), nnz))
-        return e;
+      if (begin_ain != begin_a64 || pos_ain != pos_a64)
+        if (int e = S.map_ain.build(begin_ain, pos_ain))
+          return e;
       if (int e = S.mem.get(&S.a_v, nnz))
         return e;
       if (!entry_src.empty()) {

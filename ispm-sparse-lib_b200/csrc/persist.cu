@@ -248,7 +248,6 @@ template <int V, int LP, bool WIDE> struct Group {
   template <int N> __device__ __forceinline__ void meet_sum(double (&v)[N > 0 ? N : 1])
   {
     constexpr int M = N > 0 ? N : 1;
-    constexpr int W = N > 0 ? 2 * N : 1;  // words a CTA
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     // sums over the warp's lanes; several at once share the exchanges (each
     // half of the lanes goes on with half of the sums)
@@ -513,12 +512,12 @@ template <int V, int LP, bool WIDE> struct Group {
       for (unsigned k = 0; k < nd;) {
         const unsigned left = nd - k;
         if (left >= U * np) {
-          const unsigned want = (unsigned)((1ull << (U * np)) - 1);
+          constexpr unsigned want = U * np >= 32 ? ~0u : (1u << (U * np % 32)) - 1;
           block(std::integral_constant<int, U>(),
                 live == V && k + U * np <= 32 && ((inside >> k) & want) == want, k);
           k += U * np;
         } else {
-          const unsigned want = (unsigned)((1ull << (N2 * np)) - 1);
+          constexpr unsigned want = N2 * np >= 32 ? ~0u : (1u << (N2 * np % 32)) - 1;
           block(std::integral_constant<int, N2>(),
                 live == V && left >= N2 * np && k + N2 * np <= 32 &&
                     ((inside >> k) & want) == want,

@@ -90,18 +90,14 @@ struct ispm_plan {
   ispm_slell_params mparams{};
   ispm_launch_params params{};
   double tuned = 0;
-  // element slot -> CSR entry (-1 for padding), built on the first device
-  // refresh
-  int *map = nullptr;
+  // where each slot's value comes from, built on the first device refresh
+  ispm::SlotMap map;
   long long map_n = -1;
   void drop_map()
   {
-    if (map)
-      cudaFree(map);
-    map = nullptr;
+    map.release();
     map_n = -1;
   }
-  ~ispm_plan() { drop_map(); }
 };
 
 using namespace ispm;
@@ -287,27 +283,25 @@ int ispm_plan_refresh_values(ispm_plan *p, int n_rows, const int *row_ptr, const
   if (!row_ptr || n_rows < 0)
     return fail(ISPM_ERR_INVALID, "bad CSR pattern");
   const long long nnz = row_ptr[n_rows];
-  if (!p->map || p->map_n != nnz) {
+  if (p->map.empty() || p->map_n != nnz) {
     p->drop_map();
-    std::vector<int> inv;
     try {
       std::vector<unsigned> pos;
       if (int st = value_map(p->host->m, n_rows, row_ptr, cols, pos))
         return st;
-      inv.assign((size_t)p->dev->d.meta.n_elms, -1);
-      for (size_t k = 0; k < pos.size(); k++)
-        inv[pos[k]] = (int)k;
+      if (p->dev->d.meta.n_elms != (long long)p->host->m.n_elms())
+        return fail(ISPM_ERR_INVALID, "the device matrix is not the plan's host matrix");
+      if (int st = p->map.build(slice_begins(p->host->m), pos)) {
+        p->drop_map();
+        return st;
+      }
     } catch (const std::bad_alloc &) {
+      p->drop_map();
       return fail(ISPM_ERR_NOMEM, "host allocation while mapping values");
     }
-    ISPM_CUDA_TRY(cudaMalloc(&p->map, std::max<size_t>(inv.size(), 1) * sizeof(int)));
-    if (!inv.empty())
-      ISPM_CUDA_TRY(
-          cudaMemcpy(p->map, inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice));
     p->map_n = nnz;
   }
-  // slot order: coalesced writes, reads within each slice's CSR range
-  return refresh_values_gather(p->dev->d, p->map, vals, val_dtype, (cudaStream_t)stream);
+  return refresh_slots(p->dev->d, p->map, vals, val_dtype, (cudaStream_t)stream);
 }
 
 int ispm_plan_get_params(const ispm_plan *p, ispm_slell_params *mparams,

@@ -185,18 +185,40 @@ ispm_launch_params register_walk_launch(int x_dtype, const ispm_slell_view &m,
                                         long long rows = 0);
 
 // d.elms[map[k]] = vals[k] for k < n (device arrays; vals FP32 or FP64).
-// Same from the slot side: d.elms[s] = vals[inv[s]] for every element slot
-// s (0 where inv[s] < 0); writes are coalesced, reads stay within a slice's
-// CSR range.
-int refresh_values_gather(DeviceSlell &d, const int *inv, const void *vals, int val_dtype,
-                          cudaStream_t s);
 int refresh_values(DeviceSlell &d, const unsigned *map, const void *vals, int val_dtype,
                    long long n, cudaStream_t s);
-// FP16 elements: d.elms[map[k]] = FP16(vals[k] * scale) (nearest).
-int refresh_values_f16(DeviceSlell &d, const unsigned *map, const double *vals, long long n,
-                       double scale, cudaStream_t s);
-// out = max |vals[k]| over n device values (synchronous).
-int device_absmax(const double *vals, long long n, double &out);
+
+// New values in CSR entry order for element arrays of one shape, from the slot
+// side: slices are gathered into chunks whose entries are one run of the CSR,
+// which a CTA copies through shared memory and deals out to its slots, so
+// reads and writes are whole lines and a slot costs 2 bytes of map.  A shape
+// whose slices do not cover short runs (a transposed factor) keeps the entry
+// of each slot instead and gathers.
+struct SlotMap {
+  int4 *chunk = nullptr;          // first slot, slots, first entry, entries
+  unsigned short *idx = nullptr;  // slot -> entry within its chunk (0xffff: padding)
+  int *inv = nullptr;             // slot -> entry (-1: padding), when not in chunks
+  int n_chunks = 0, max_entries = 0;
+  long long n_slots = 0;
+  SlotMap() = default;
+  SlotMap(const SlotMap &) = delete;
+  SlotMap &operator=(const SlotMap &) = delete;
+  ~SlotMap() { release(); }
+  void release();
+  bool empty() const { return !chunk && !inv; }
+  // slice_begin: first slot of every slice and the slot count; pos: entry ->
+  // slot.
+  int build(const std::vector<unsigned> &slice_begin, const std::vector<unsigned> &pos);
+};
+// First slot of every slice of h, and its slot count.
+std::vector<unsigned> slice_begins(const HostSlell &h);
+// d.elms (and second->elms, of the same shape) = vals in the map's order, 0 on
+// padding.  amax (FP16 elements; device): values times the power of two that
+// maps *amax into [2^13, 2^14).
+int refresh_slots(DeviceSlell &d, const SlotMap &map, const void *vals, int val_dtype,
+                  cudaStream_t s, DeviceSlell *second = nullptr, const double *amax = nullptr);
+// *out = max |vals[k]| over n device values (device result; 0 for n = 0).
+int absmax_async(const double *vals, long long n, double *out, cudaStream_t s);
 
 }  // namespace ispm
 
