@@ -33,6 +33,7 @@
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "cuda_util.cuh"
@@ -844,10 +845,14 @@ int set_smem_attrs()
 
 struct ispm_mlp {
   float *prm = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr;
+  float *host = nullptr;  // pinned: results on their way to the caller (kPart floats)
+  mutable std::mutex host_mu;
   int part_cta = 0;
   int step = 0;
   ~ispm_mlp()
   {
+    if (host)
+      cudaFreeHost(host);
     for (float *p : {prm, m, v, grad, part})
       if (p)
         cudaFree(p);
@@ -877,6 +882,10 @@ int ispm_mlp_create(const float *init_params, ispm_mlp **out)
     ISPM_CUDA_TRY(cudaMemset(*pp, 0, sizeof(float) * kPart));
   }
   ISPM_CUDA_TRY(cudaMemcpy(h->prm, init_params, sizeof(float) * kParams, cudaMemcpyHostToDevice));
+  if (cudaMallocHost(&h->host, sizeof(float) * kPart) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(ISPM_ERR_NOMEM, "pinned host allocation");
+  }
   if (int e = set_smem_attrs())
     return e;
   *out = h.release();
@@ -888,7 +897,10 @@ int ispm_mlp_get_params(const ispm_mlp *m, float *host_out)
   clear_error();
   if (!m || !host_out)
     return fail(ISPM_ERR_INVALID, "NULL argument");
-  ISPM_CUDA_TRY(cudaMemcpy(host_out, m->prm, sizeof(float) * kParams, cudaMemcpyDeviceToHost));
+  std::lock_guard<std::mutex> lock(m->host_mu);
+  ISPM_CUDA_TRY(cudaMemcpyAsync(m->host, m->prm, sizeof(float) * kParams, cudaMemcpyDeviceToHost, 0));
+  ISPM_CUDA_TRY(cudaStreamSynchronize(0));
+  memcpy(host_out, m->host, sizeof(float) * kParams);
   return ISPM_OK;
 }
 
@@ -954,16 +966,16 @@ int ispm_mlp_loss_grad(ispm_mlp *m, long long n_rows, const void *feat_bf16,
   ISPM_CUDA_TRY(launch_kernel(mlp_reduce_kernel, dim3((kPart + 31) / 32), dim3(32 * kReduceWarps), 0,
                               s, true, (const float *)m->part, grid, m->grad));
   ISPM_CUDA_TRY(cudaPeekAtLastError());
-  if (grad_out)
-    ISPM_CUDA_TRY(cudaMemcpyAsync(grad_out, m->grad, sizeof(float) * kParams,
+  if (grad_out || loss_out) {  // one copy: the loss sits behind the gradient
+    std::lock_guard<std::mutex> lock(m->host_mu);
+    const size_t from = grad_out ? 0 : kParams;
+    ISPM_CUDA_TRY(cudaMemcpyAsync(m->host + from, m->grad + from, sizeof(float) * (kPart - from),
                                   cudaMemcpyDeviceToHost, s));
-  if (loss_out) {
-    float l = 0.f;
-    ISPM_CUDA_TRY(cudaMemcpyAsync(&l, m->grad + kParams, sizeof(float), cudaMemcpyDeviceToHost, s));
     ISPM_CUDA_TRY(cudaStreamSynchronize(s));
-    *loss_out = l;
-  } else if (grad_out) {
-    ISPM_CUDA_TRY(cudaStreamSynchronize(s));
+    if (grad_out)
+      memcpy(grad_out, m->host, sizeof(float) * kParams);
+    if (loss_out)
+      *loss_out = m->host[kParams];
   }
   return ISPM_OK;
 }

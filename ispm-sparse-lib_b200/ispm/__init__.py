@@ -124,6 +124,7 @@ def _declare(L):
         "ispm_plan_upload": (i, [vp]),
         "ispm_plan_update_device_matrix_coefs": (i, [vp]),
         "ispm_plan_change_host_matrix": (i, [vp, i, i, vp, vp, vp]),
+        "ispm_plan_refresh_values": (i, [vp, i, vp, vp, vp, i, vp]),
         "ispm_plan_get_params": (i, [vp, C.POINTER(slell_params),
                                      C.POINTER(spmv_launch_params)]),
         "ispm_plan_host_matrix": (vp, [vp]),
@@ -163,28 +164,34 @@ def _check(status: int):
 
 def _ptr(a):
     """Address of a numpy array, torch tensor or raw int pointer."""
+    address = getattr(a, "data_ptr", None)  # torch: the common case, so first
+    if address is not None:
+        return address()
     if a is None:
         return None
     if isinstance(a, int):
         return a
     if isinstance(a, np.ndarray):
         return a.ctypes.data
-    if hasattr(a, "data_ptr"):
-        return a.data_ptr()
     raise TypeError(f"cannot take the address of {type(a)}")
 
 
+_DTYPE_CODES = {}  # numpy / torch dtype -> F32 / F64 (naming a dtype costs a microsecond)
+
+
 def _dtype_code(a) -> int:
-    if isinstance(a, np.ndarray):
-        dt = a.dtype
-    else:
-        dt = getattr(a, "dtype", None)
-    s = str(dt)
-    if s.endswith("float32"):
-        return F32
-    if s.endswith("float64"):
-        return F64
-    raise TypeError(f"unsupported element type {dt}")
+    dt = getattr(a, "dtype", None)
+    code = _DTYPE_CODES.get(dt)
+    if code is None:
+        s = str(dt)
+        if s.endswith("float32"):
+            code = F32
+        elif s.endswith("float64"):
+            code = F64
+        else:
+            raise TypeError(f"unsupported element type {dt}")
+        _DTYPE_CODES[dt] = code
+    return code
 
 
 def _stream(stream):
@@ -555,7 +562,10 @@ class spmv_plan:
             self._h = None
 
     def execute_spmv(self, x, y, stream=None):
-        _check(_lib().ispm_plan_execute(self._h, _ptr(x), _ptr(y), _stream(stream)))
+        status = _L.ispm_plan_execute(self._h, _ptr(x), _ptr(y),
+                                      None if stream is None else _stream(stream))
+        if status:
+            _check(status)
 
     def upload(self):
         _check(_lib().ispm_plan_upload(self._h))
@@ -905,12 +915,8 @@ def slell_value_map(m: slell_matrix, A: csr_matrix) -> np.ndarray:
 def plan_refresh_values(plan: "spmv_plan", A: csr_matrix, vals_dev, stream=None):
     """Scatter new CSR values (device array, A's pattern) into the plan's device
     matrix (ispm_plan_refresh_values)."""
-    L = _lib()
-    vp = C.c_void_p
-    L.ispm_plan_refresh_values.argtypes = [vp, C.c_int, vp, vp, vp, C.c_int, vp]
-    L.ispm_plan_refresh_values.restype = C.c_int
     n_src = A.row_ptr.size - 1
-    _check(L.ispm_plan_refresh_values(plan._h, n_src, _ptr(A.row_ptr), _ptr(A.cols),
+    _check(_lib().ispm_plan_refresh_values(plan._h, n_src, _ptr(A.row_ptr), _ptr(A.cols),
                                       _ptr(vals_dev), _dtype_code(vals_dev), _stream(stream)))
 
 

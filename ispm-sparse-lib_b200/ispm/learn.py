@@ -73,9 +73,15 @@ def _declare():
     _DECLARED = True
 
 
+_N_PARAMS = None
+
+
 def n_params() -> int:
-    _declare()
-    return int(_lib().ispm_mlp_n_params())
+    global _N_PARAMS
+    if _N_PARAMS is None:
+        _declare()
+        _N_PARAMS = int(_lib().ispm_mlp_n_params())
+    return _N_PARAMS
 
 
 def init_params(seed: int = 0) -> np.ndarray:
@@ -109,7 +115,7 @@ class MLP:
             self._h = None
 
     def params(self) -> np.ndarray:
-        out = np.zeros(n_params(), np.float32)
+        out = np.empty(n_params(), np.float32)
         _check(_lib().ispm_mlp_get_params(self._h, _ptr(out)))
         return out
 
@@ -127,7 +133,7 @@ class MLP:
 
     def loss_grad(self, feat, target, weight=None, stream=None, want_grad=True):
         loss = C.c_double()
-        g = np.zeros(n_params(), np.float32) if want_grad else None
+        g = np.empty(n_params(), np.float32) if want_grad else None
         _check(_lib().ispm_mlp_loss_grad(self._h, feat.shape[0], _ptr(feat), _ptr(target),
                                          _ptr(weight), _ptr(g), C.byref(loss),
                                          _stream(stream)))
