@@ -35,14 +35,15 @@ constexpr int kMaxPattern = 32;
 
 // One factor row per group of G lanes (G = 4, 8, 16 or 32, the smallest that
 // holds the longest pattern), 32 / G rows a warp; lane l owns row l of the
-// local matrix in registers.
+// local matrix in registers, KM columns of it (the longest pattern, rounded
+// up).
 //
-// What bounds it: shared-memory and L1 wavefronts (83% of their rate on the
-// 72^3 27-point matrix, issue slots 67%, DRAM 4%).  A row of that stencil (K =
+// What bounds it: shared-memory and L1 wavefronts (81% of their rate on the
+// 72^3 27-point matrix, issue slots 68%, DRAM 4%).  A row of that stencil (K =
 // 14) needs about 110 FP64 multiply-adds a lane fed by shared-memory
 // broadcasts, and its 14 x 14 local matrix comes from 14 rows of A that
 // neighbouring factor rows share through L1; the bytes (12 per entry of A, 8
-// per entry of G) are a fraction of that time.  373,248 rows take 0.46 ms;
+// per entry of G) are a fraction of that time.  373,248 rows take 0.44 ms;
 // one warp a row with a walk per lane, a Cholesky factorization in shared
 // memory and a serial back-substitution took 3.39 ms.  So:
 //  * the group reads each row of A it needs as one coalesced run (the entries
@@ -55,7 +56,7 @@ constexpr int kMaxPattern = 32;
 //  * the last row of L^-1, z = L^-T e, is all that the factor row needs
 //    (g = z / sqrt(d_last)): one lane-parallel back-substitution, reading the
 //    stored columns.
-template <int G>
+template <int G, int KM>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     fsai_rows_kernel(int n, const int *__restrict__ a_rp, const int *__restrict__ a_ci,
                      const double *__restrict__ a_v, const int *__restrict__ g_rp,
@@ -102,8 +103,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     }
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      int e = __shfl_sync(full, start, c0 + q, G) + lane;
-      const int end = __shfl_sync(full, stop, c0 + q, G);
+      int e = 0, end = -1;  // (formed when a run goes on past the group)
       for (;;) {
         if (col[q] <= i) {
           int at = 0;
@@ -116,6 +116,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         // a longer run: on while its last entry is still left of column i
         if (!__any_sync(full, lane == G - 1 && col[q] < i))
           break;
+        if (end < 0) {
+          e = __shfl_sync(full, start, c0 + q, G) + lane;
+          end = __shfl_sync(full, stop, c0 + q, G);
+        }
         e += G;
         const bool in = col[q] < i && e < end;
         col[q] = in ? __ldg(a_ci + e) : kNone;
@@ -124,23 +128,23 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     }
   }
   __syncwarp();
-  double a[G];
+  double a[KM];
 #pragma unroll
-  for (int k = 0; k < G; k += 2) {
+  for (int k = 0; k < KM; k += 2) {
     const double2 v = *reinterpret_cast<const double2 *>(&S[lane][k]);
     a[k] = v.x;
     a[k + 1] = v.y;
   }
   if (lane >= K) {  // identity past the pattern
 #pragma unroll
-    for (int k = 0; k < G; k++)
+    for (int k = 0; k < KM; k++)
       a[k] = k == lane ? 1.0 : 0.0;
   }
   __syncwarp();
   bool ok = true;
   double rd_own = 1.0, d_own = 1.0;
 #pragma unroll
-  for (int k = 0; k < G; k++) {
+  for (int k = 0; k < KM; k++) {
     if (k < kw) {
       S[k][lane] = a[k];  // column k, unscaled (the lanes k .. are read)
       __syncwarp();
@@ -153,14 +157,18 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       }
       const double l = a[k] * rd;
 #pragma unroll
-      for (int j = k + 1; j < G; j++)
-        a[j] = fma(-l, S[k][j], a[j]);
+      for (int j = (k + 1) & ~1; j < KM; j += 2) {
+        const double2 u = *reinterpret_cast<const double2 *>(&S[k][j]);
+        if (j > k)
+          a[j] = fma(-l, u.x, a[j]);
+        a[j + 1] = fma(-l, u.y, a[j + 1]);
+      }
     }
   }
   __syncwarp();
   double s = 0.0, z = lane == K - 1 ? 1.0 : 0.0;
 #pragma unroll
-  for (int c = G - 1; c > 0; c--) {
+  for (int c = KM - 1; c > 0; c--) {
     if (c < kw) {
       const double zc = __shfl_sync(full, z, c, G);
       s = fma(S[lane][c], zc, s);  // used by the lanes left of c alone
@@ -182,12 +190,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   }
 }
 
-template <int G>
+template <int G, int KM>
 void launch_rows(int n, const int *a_rp, const int *a_ci, const double *a_v, const int *g_rp,
                  double *g_v, unsigned *fb, cudaStream_t s)
 {
   const int rows = kWarpsPerBlock * (32 / G);
-  fsai_rows_kernel<G><<<(n + rows - 1) / rows, kWarpsPerBlock * 32, 0, s>>>(n, a_rp, a_ci, a_v,
+  fsai_rows_kernel<G, KM><<<(n + rows - 1) / rows, kWarpsPerBlock * 32, 0, s>>>(n, a_rp, a_ci, a_v,
                                                                             g_rp, g_v, fb);
 }
 
@@ -255,14 +263,27 @@ int fsai_build_values(int n, int max_pattern, const int *a_rp_d, const int *a_ci
   if (max_pattern > kMaxPattern)
     return fail(ISPM_ERR_INVALID, "FSAI pattern of %d entries (at most %d)", max_pattern,
                 kMaxPattern);
-  if (max_pattern <= 4)
-    launch_rows<4>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
-  else if (max_pattern <= 8)
-    launch_rows<8>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
-  else if (max_pattern <= 16)
-    launch_rows<16>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
-  else
-    launch_rows<32>(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
+  const auto rows = [](int k) {
+    switch ((k + 1) / 2) {
+    case 0:
+    case 1:
+    case 2: return launch_rows<4, 4>;
+    case 3: return launch_rows<8, 6>;
+    case 4: return launch_rows<8, 8>;
+    case 5: return launch_rows<16, 10>;
+    case 6: return launch_rows<16, 12>;
+    case 7: return launch_rows<16, 14>;
+    case 8: return launch_rows<16, 16>;
+    case 9:
+    case 10: return launch_rows<32, 20>;
+    case 11:
+    case 12: return launch_rows<32, 24>;
+    case 13:
+    case 14: return launch_rows<32, 28>;
+    default: return launch_rows<32, 32>;
+    }
+  }(max_pattern);
+  rows(n, a_rp_d, a_ci_d, a_v_d, g_rp_d, g_v_d, fallbacks_d, s);
   cudaError_t e = cudaPeekAtLastError();
   return e == cudaSuccess ? ISPM_OK : fail(ISPM_ERR_CUDA, "fsai rows: %s", cudaGetErrorString(e));
 }
