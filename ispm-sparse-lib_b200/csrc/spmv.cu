@@ -455,6 +455,118 @@ __global__ void __launch_bounds__(1024) slell_spmv_kernel(SpmvArgs<T, E> a)
   spmv_body<T, E, H, W, VAR, DIAG, false>(a, blockIdx.x);
 }
 
+// Diagonal blocks of fixed height, no more than one thread a row: a warp takes
+// 32 V consecutive rows of a slice, lane l rows l, l + 32, ..., so a diagonal's
+// column and addresses serve V rows, every load is a line of consecutive words
+// whatever the window's alignment, and UV / V diagonals' loads are in flight
+// together.  The same sums in the same order as the walk of consecutive rows
+// (spmv_body), whose FP64 windows take two loads a step and whose long threads
+// leave a last wave nearly empty.  Which of the two: strided_rows() below.
+// What bounds it is DRAM where the matrix is larger than L2 (27-point 128^3 FP64
+// on FP32: 60.5 us, 4.1 TB/s; 74.7 before) and the latency of the loads in flight
+// where it is not.  Tail: the diagonals past the last whole block in one masked
+// block, not one by one (fewer round trips, more registers).  Two: the loads that
+// need no bounds check compiled as a copy of their own (48 to 64 registers a
+// thread, not 60 to 100).
+template <class T, class E, int V, int UV, bool Tail, bool Two>
+__global__ void __launch_bounds__(256) slell_strided_kernel(SpmvArgs<T, E> a)
+{
+  constexpr unsigned full = 0xffffffffu;
+  constexpr int U = UV / V;  // diagonals a block
+  pdl_wait();
+  if (a.skip && *a.skip)
+    return;
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned tile = blockIdx.x * (256 / 32) + (threadIdx.x >> 5);
+  const unsigned S = a.slice_height, lh = 31 - __clz(S), n = a.n_cols;
+  const unsigned base = tile * (32 * V), slice = base >> lh;
+  if (slice >= a.n_slices)
+    return;
+  const unsigned r = (base & (S - 1)) + lane;
+  const unsigned *rec = a.sp + 3 * (size_t)slice;
+  const unsigned e0 = __ldg(rec), c0 = __ldg(rec + 1), d0 = __ldg(rec + 2);
+  const unsigned e1 = __ldg(rec + 3), c1 = __ldg(rec + 4);
+  const unsigned nc = (c1 - c0) >> lh, nd = ((e1 - e0) >> lh) - nc;
+  const T *__restrict__ x = a.x;
+  T acc[V];
+#pragma unroll
+  for (int v = 0; v < V; v++)
+    acc[v] = T(0);
+  const E *e = a.elms + e0 + r;
+  const unsigned *cc = a.cols + c0 + r;
+#pragma unroll 2
+  for (unsigned k = 0; k < nc; k++, e += S, cc += S)
+#pragma unroll
+    for (int v = 0; v < V; v++)
+      acc[v] = fma(T(__ldcs(e + 32 * v)), ld_x_guard(x, __ldcs(cc + 32 * v), n), acc[v]);
+  for (unsigned kb = 0; kb < nd; kb += 32) {
+    const unsigned m = min(32u, nd - kb);
+    const unsigned pos = lane < m ? __ldg(a.sp + d0 + kb + lane) - S + (base & (S - 1)) : 0u;
+    const unsigned inside = __ballot_sync(full, lane < m && pos < n && n - pos >= 32u * V);
+    // N diagonals from the k-th on (the masked tail: those left)
+    auto block = [&](auto width, auto tail, bool whole, unsigned k) {
+      constexpr int N = decltype(width)::value;
+      constexpr bool Masked = decltype(tail)::value;
+      E ev[N][V];
+      T xv[N][V];
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        if (Masked && k + u >= m)
+          continue;
+        const unsigned c = __shfl_sync(full, pos, k + u) + lane;
+        const E *ep = e + ((k + u) << lh);
+        if (whole) {
+          const T *xp = x + c;
+#pragma unroll
+          for (int v = 0; v < V; v++) {
+            ev[u][v] = __ldcs(ep + 32 * v);
+            xv[u][v] = __ldg(xp + 32 * v);
+          }
+        } else {
+#pragma unroll
+          for (int v = 0; v < V; v++) {
+            ev[u][v] = __ldcs(ep + 32 * v);
+            xv[u][v] = ld_x_guard(x, c + 32u * v, n);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        if (Masked && k + u >= m)
+          continue;
+#pragma unroll
+        for (int v = 0; v < V; v++)
+          acc[v] = fma(T(ev[u][v]), xv[u][v], acc[v]);
+      }
+    };
+    constexpr unsigned want = U >= 32 ? ~0u : (1u << (U & 31)) - 1;
+    using Whole = std::integral_constant<int, U>;
+    unsigned k = 0;
+    auto blocks = [&](auto width, auto tail, bool whole, unsigned k) {
+      if (!Two)
+        block(width, tail, whole, k);
+      else if (whole)
+        block(width, tail, true, k);
+      else
+        block(width, tail, false, k);
+    };
+    for (; k + U <= m; k += U)
+      blocks(Whole(), std::false_type(), ((inside >> k) & want) == want, k);
+    if constexpr (Tail) {
+      if (k < m)
+        blocks(Whole(), std::true_type(), (inside >> k) == (full >> (32 - (m - k))), k);
+    } else {
+      for (; k < m; k++)
+        block(std::integral_constant<int, 1>(), std::false_type(), false, k);
+    }
+    e += m << lh;
+  }
+  pdl_trigger();
+#pragma unroll
+  for (int v = 0; v < V; v++)
+    a.y[base + lane + 32 * v] = acc[v];
+}
+
 // Lane-segmented products of up to kMaxLaneOps operators in one launch: CTAs
 // first[k] .. first[k + 1] - 1 serve operator k.  Operators of one kind
 // (rows a thread, hblock width, diagonal blocks, CTA size) share a launch
@@ -553,6 +665,97 @@ int launch_h(const SpmvArgs<T, E> &args, const ispm_slell_view &m, unsigned tps,
   return fail(ISPM_ERR_INVALID, "hblock %u", m.hblock);
 }
 
+// The most rows a thread of the strided walk may take for this launch, 0 for
+// the walk of consecutive rows.  Us, strided / consecutive, cubes of side n:
+//  * FP64 vectors on FP32 elements: always, and also where the walk has several
+//    threads a row, if the rows are short and their columns diagonals (a long
+//    row or a long list of columns needs its threads).  7-point n = 16 3.6 / 4.0,
+//    55 3.9 / 7.9, 76 5.4 / 11.2, 105 9.5 / 16.8, 128 19.5 / 29.5; 27-point
+//    n = 28 4.0 / 5.4, 64 9.1 / 15.0, 90 23.0 / 36.4, 128 60.5 / 74.7.
+//  * FP64 elements, one thread a row: 7-point n = 70 5.7 / 7.2, 90 9.2 / 13.0, 120
+//    21.7 / 25.4.  Slices below 128 rows: not where the last wave of the two-row
+//    threads is nearly full: 27-point n = 70 15.1 / 19.2, 80 21.4 / 22.1, 90 29.0 /
+//    37.9, but 105 47.5 / 46.4, 120 72.0 / 69.0.
+//  * FP32 vectors, one thread a row, slices of 256 rows: 7-point n = 90 6.2 / 8.2,
+//    112 11.1 / 13.5, 128 14.2 / 15.9.  Shorter slices: where the four-row threads
+//    are more than one wave and at most one and a half: 27-point n = 110 32.9 /
+//    42.1, 122 43.6 / 47.0, but 96 22.0 / 21.9, 126 49.6 / 47.0.
+int strided_rows(const ispm_launch_params &p, const ispm_slell_view &m, size_t vec_size)
+{
+  const unsigned S = m.slice_height;
+  if (!m.diags || m.var_height || m.hblock != 1 || S < 64 || p.N * p.H < S || p.H < 2)
+    return 0;
+  const int most = S >= 256 ? 8 : S >= 128 ? 4 : 2;
+  const double rows = (double)m.n_slices * S, sms = device_sm_count();
+  if (vec_size == 8 && m.elm_dtype == ISPM_F32)
+    return p.N * p.H == S || (m.n_elms <= 32ll * m.n_rows && 8 * m.n_cols_arr <= m.n_elms)
+               ? most
+               : 0;
+  if (p.N * p.H > S)
+    return 0;
+  if (vec_size == 8) {
+    const double waves = rows / (2 * 1024 * sms);
+    return most > 2 || waves - std::floor(waves) <= 0.75 ? std::min(most, 4) : 0;
+  }
+  const double waves = rows / (4 * 2048 * sms);
+  return most == 8 || (waves > 1.0 && waves <= 1.5) ? most : 0;
+}
+
+// One shape of the strided walk; false, and no launch, where one_wave is asked
+// for and its blocks are not all resident at once.
+template <class T, class E, int V, int UV, bool Tail, bool Two>
+bool launch_strided(const SpmvArgs<T, E> &a, bool one_wave, cudaStream_t s, cudaError_t &e)
+{
+  auto kernel = slell_strided_kernel<T, E, V, UV, Tail, Two>;
+  const unsigned tiles = a.n_slices * (a.slice_height / (32 * V)), grid = (tiles + 7) / 8;
+  if (one_wave) {
+    static const int per_sm = [&] {
+      int b = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 256, 0) != cudaSuccess)
+        b = 0;
+      return b;
+    }();
+    if (grid > (unsigned)per_sm * device_sm_count())
+      return false;
+  }
+  e = launch_kernel(kernel, dim3(grid), dim3(256), 0, s, a.pdl != 0, a);
+  if (e == cudaSuccess)
+    e = cudaPeekAtLastError();
+  return true;
+}
+
+// The first shape of each list whose blocks are all resident, past them the last.
+// Rows x loads in flight, us: FP64 on FP32, 7-point 64^3 2 x 12 4.0, 4 x 8 4.8;
+// 76^3 4 x 8 5.4, 2 x 12 6.7; 98^3 8 x 16 8.7, 4 x 8 9.7; 27-point 28^3 1 x 16 4.0,
+// 2 x 12 6.3; 64^3 2 x 12 9.1, 2 x 8 9.8; 70^3 2 x 8 12.2, 2 x 12 15.1.
+template <class T, class E>
+int launch_strided(const SpmvArgs<T, E> &a, int most, cudaStream_t s)
+{
+  cudaError_t e = cudaSuccess;
+  if constexpr (sizeof(T) == 8 && sizeof(E) == 4)
+    launch_strided<T, E, 1, 16, true, true>(a, true, s, e) ||
+        launch_strided<T, E, 2, 12, true, false>(a, true, s, e) ||
+        launch_strided<T, E, 2, 12, false, false>(a, true, s, e) ||
+        (most == 2 ? launch_strided<T, E, 2, 8, false, true>(a, true, s, e) ||
+                         launch_strided<T, E, 2, 12, false, false>(a, false, s, e)
+                   : launch_strided<T, E, 4, 8, true, false>(a, true, s, e) ||
+                         launch_strided<T, E, 4, 8, false, true>(a, most == 8, s, e) ||
+                         launch_strided<T, E, 8, 16, false, true>(a, false, s, e));
+  else if constexpr (sizeof(T) == 8)
+    most == 2 ? launch_strided<T, E, 2, 8, false, true>(a, true, s, e) ||
+                    launch_strided<T, E, 2, 8, false, false>(a, false, s, e)
+              : launch_strided<T, E, 4, 8, true, false>(a, true, s, e) ||
+                    launch_strided<T, E, 4, 8, false, true>(a, true, s, e) ||
+                    launch_strided<T, E, 4, 8, false, false>(a, false, s, e);
+  else
+    most == 8 ? launch_strided<T, E, 4, 8, true, false>(a, true, s, e) ||
+                    launch_strided<T, E, 8, 16, false, false>(a, false, s, e)
+    : most == 4 ? launch_strided<T, E, 4, 16, false, true>(a, false, s, e)
+                : launch_strided<T, E, 2, 16, false, true>(a, false, s, e);
+  return e == cudaSuccess ? ISPM_OK
+                          : fail(ISPM_ERR_CUDA, "SpMV launch: %s", cudaGetErrorString(e));
+}
+
 // The arguments every launch of matrix m shares.
 template <class T, class E>
 int fill_args(SpmvArgs<T, E> &a, const ispm_launch_params &p, const ispm_slell_view &m,
@@ -617,6 +820,9 @@ int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void 
       return launch_staged<E>(a, si, s);
     }
   }
+  if constexpr (std::is_same<E, float>::value || std::is_same<E, double>::value)
+    if (const int most = strided_rows(p, m, sizeof(T)); most && !(ep && ep->out))
+      return launch_strided<T, E>(a, most, s);
   switch (p.H) {
   case 1: return launch_h<T, E, 1>(a, m, p.N, s);
   case 2: return launch_h<T, E, 2>(a, m, p.N, s);
