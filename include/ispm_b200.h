@@ -372,7 +372,8 @@ typedef struct {
                            as 1): the chunk is the body of the graph's while
                            node, repeated on the device until the flags end
                            the phase, so a phase is one graph launch and one
-                           host wait; 0: eager launches */
+                           host wait; 0: eager launches.  A system small enough
+                           for L2 is solved in one launch, whatever this says */
   double replace_ratio_f32; /* reliable update once the recursive residual fell by
                                this factor since the last one (FP32 inner) */
   double replace_ratio_f64; /* same for FP64 */

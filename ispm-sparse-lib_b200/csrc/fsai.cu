@@ -15,8 +15,8 @@
 // of seconds.
 //
 // A group of lanes per row gathers the |P_i| x |P_i| local matrix (|P_i| <=
-// 32), factors it (L D L^T) and back-substitutes.  FP64 throughout.  A local matrix that is not positive definite (indefinite A)
-// falls back to the Jacobi row e_i / sqrt(a_ii) when a_ii > 0, else to e_i,
+// 32), factors it (L D L^T) and back-substitutes.  FP64 throughout.  A local
+// matrix that is not positive definite (indefinite A) falls back to the Jacobi row e_i / sqrt(a_ii) when a_ii > 0, else to e_i,
 // and is counted.
 #include <cuda_runtime.h>
 
