@@ -678,8 +678,9 @@ int launch_h(const SpmvArgs<T, E> &args, const ispm_slell_view &m, unsigned tps,
 //    37.9, but 105 47.5 / 46.4, 120 72.0 / 69.0.
 //  * FP32 vectors, one thread a row, slices of 256 rows: 7-point n = 90 6.2 / 8.2,
 //    112 11.1 / 13.5, 128 14.2 / 15.9.  Shorter slices: where the four-row threads
-//    are more than one wave and at most one and a half: 27-point n = 110 32.9 /
-//    42.1, 122 43.6 / 47.0, but 96 22.0 / 21.9, 126 49.6 / 47.0.
+//    are at most 0.8 of a wave (too few loads in flight) or one to one and a half
+//    (a last wave nearly empty): 27-point n = 85 18.3 / 27.9, 97 21.7 / 29.3, 110
+//    30.3 / 42.2, 122 41.3 / 47.0, but 104 26.6 / 24.1, 128 47.3 / 44.9.
 int strided_rows(const ispm_launch_params &p, const ispm_slell_view &m, size_t vec_size)
 {
   const unsigned S = m.slice_height;
@@ -698,7 +699,7 @@ int strided_rows(const ispm_launch_params &p, const ispm_slell_view &m, size_t v
     return most > 2 || waves - std::floor(waves) <= 0.75 ? std::min(most, 4) : 0;
   }
   const double waves = rows / (4 * 2048 * sms);
-  return most == 8 || (waves > 1.0 && waves <= 1.5) ? most : 0;
+  return most == 8 || waves <= 0.8 || (waves > 1.0 && waves <= 1.5) ? most : 0;
 }
 
 // One shape of the strided walk; false, and no launch, where one_wave is asked
@@ -750,8 +751,8 @@ int launch_strided(const SpmvArgs<T, E> &a, int most, cudaStream_t s)
   else
     most == 8 ? launch_strided<T, E, 4, 8, true, false>(a, true, s, e) ||
                     launch_strided<T, E, 8, 16, false, false>(a, false, s, e)
-    : most == 4 ? launch_strided<T, E, 4, 16, false, true>(a, false, s, e)
-                : launch_strided<T, E, 2, 16, false, true>(a, false, s, e);
+    : most == 4 ? launch_strided<T, E, 4, 8, false, false>(a, false, s, e)
+                : launch_strided<T, E, 2, 8, false, false>(a, false, s, e);
   return e == cudaSuccess ? ISPM_OK
                           : fail(ISPM_ERR_CUDA, "SpMV launch: %s", cudaGetErrorString(e));
 }
