@@ -231,6 +231,19 @@ int ispm_slell_value_map(const ispm_slell *m, int n_rows, const int *row_ptr, co
                          unsigned *map);
 int ispm_dslell_refresh_values(ispm_dslell *d, const unsigned *map_dev, const void *vals_dev,
                                int val_dtype, int n_nz, void *stream);
+/* How a refresh deals out a matrix's slots (host only, for inspection): slices
+ * that start at slots slice_begin[0 .. n_slices] and hold CSR entries
+ * first_entry[s] .. last_entry[s] (first > last: padding alone) in chunks of
+ * neighbouring slices, `entries` CSR entries from `entry` on into `slots`
+ * slots from `first` on.  Returns the count (writes at most cap), 0 where a
+ * slice's run is too long for a chunk (every slot is then gathered by itself),
+ * -1 for bad arguments. */
+typedef struct {
+  unsigned first, slots;
+  int entry, entries;
+} ispm_refresh_chunk;
+int ispm_refresh_chunks(int n_slices, const unsigned *slice_begin, const int *first_entry,
+                        const int *last_entry, ispm_refresh_chunk *out, int cap);
 int ispm_plan_get_params(const ispm_plan *p, ispm_slell_params *mparams,
                          ispm_launch_params *params);
 /* The plan's matrices (NULL if absent); owned by the plan. */

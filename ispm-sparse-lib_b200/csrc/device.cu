@@ -365,16 +365,22 @@ __device__ __forceinline__ double f16_scale(const double *amax)
 template <class E, class E2, class V>
 __global__ void __launch_bounds__(256)
     refresh_chunks_kernel(E *__restrict__ elms, E2 *__restrict__ second,
-                          const int4 *__restrict__ chunk, const unsigned short *__restrict__ idx,
-                          const V *__restrict__ vals, const double *amax)
+                          const SlotChunk *__restrict__ chunk,
+                          const unsigned short *__restrict__ idx, const V *__restrict__ vals,
+                          const double *amax)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V *sm = reinterpret_cast<V *>(smem_raw);
   pdl_wait();
-  const int4 c = __ldg(chunk + blockIdx.x);
+  const uint4 c = __ldg(reinterpret_cast<const uint4 *>(chunk) + blockIdx.x);
   const V *v = vals + c.z;
+  const int slots = (int)c.y, entries = (int)c.w;
+  elms += c.x;
+  idx += c.x;
+  if (second)
+    second += c.x;
 #pragma unroll 8
-  for (int i = threadIdx.x; i < c.w; i += 256)
+  for (int i = threadIdx.x; i < entries; i += 256)
     sm[i] = __ldcs(v + i);
   const double scale = f16_scale(amax);
   __syncthreads();
@@ -387,23 +393,23 @@ __global__ void __launch_bounds__(256)
       E2 v[4];
     };
 #pragma unroll 2
-    for (int i = 4 * threadIdx.x; i < c.y; i += 1024) {
-      const ushort4 k = __ldcs(reinterpret_cast<const ushort4 *>(idx + c.x + i));
+    for (int i = 4 * threadIdx.x; i < slots; i += 1024) {
+      const ushort4 k = __ldcs(reinterpret_cast<const ushort4 *>(idx + i));
       const double a = value(k.x), b = value(k.y), d = value(k.z), e = value(k.w);
-      *reinterpret_cast<Q *>(elms + c.x + i) =
+      *reinterpret_cast<Q *>(elms + i) =
           Q{{element<E>(a, scale), element<E>(b, scale), element<E>(d, scale),
              element<E>(e, scale)}};
       if (second)
-        *reinterpret_cast<Q2 *>(second + c.x + i) =
+        *reinterpret_cast<Q2 *>(second + i) =
             Q2{{element<E2>(a, scale), element<E2>(b, scale), element<E2>(d, scale),
                 element<E2>(e, scale)}};
     }
   } else {
-    for (int i = threadIdx.x; i < c.y; i += 256) {
-      const double a = value(idx[c.x + i]);
-      elms[c.x + i] = element<E>(a, scale);
+    for (int i = threadIdx.x; i < slots; i += 256) {
+      const double a = value(idx[i]);
+      elms[i] = element<E>(a, scale);
       if (second)
-        second[c.x + i] = element<E2>(a, scale);
+        second[i] = element<E2>(a, scale);
     }
   }
   pdl_trigger();
@@ -448,11 +454,44 @@ void SlotMap::release()
   n_slots = 0;
 }
 
-int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<unsigned> &pos)
+std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
+                                   const std::vector<int2> &span)
 {
   // a chunk: slices up to 3,072 entries (24 KB of FP64 values, eight CTAs an
-  // SM), a taller slice alone up to 8,192
+  // SM), a taller slice alone up to 8,192; no more than 2^30 slots, so that a
+  // slot's place in its chunk is an int
   constexpr int kFull = 3072, kMost = 8192;
+  constexpr unsigned kSlots = 1u << 30;
+  std::vector<SlotChunk> ch;
+  int lo = 0, hi = -1;  // the open chunk's entries
+  unsigned first = 0;
+  auto close = [&](unsigned end) {
+    const int n = hi >= lo ? hi - lo + 1 : 0;
+    while (first < end) {
+      const unsigned slots = std::min(end - first, kSlots);
+      ch.push_back(SlotChunk{first, slots, n ? lo : 0, n});
+      first += slots;
+    }
+    lo = 0;
+    hi = -1;
+  };
+  for (size_t s = 0; s < span.size(); s++) {
+    const int l = span[s].x, h = span[s].y;
+    if (h < l)
+      continue;  // (padding alone joins the open chunk)
+    if (h - l >= kMost)
+      return {};
+    if (hi >= lo && std::max(hi, h) - std::min(lo, l) >= kFull)
+      close(slice_begin[s]);
+    lo = hi >= lo ? std::min(lo, l) : l;
+    hi = std::max(hi, h);
+  }
+  close(slice_begin.back());
+  return ch;
+}
+
+int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<unsigned> &pos)
+{
   release();
   n_slots = slice_begin.back();
   std::vector<int> in((size_t)n_slots, -1);
@@ -473,49 +512,26 @@ int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<u
       span[(size_t)s] = make_int2(l, h);
     }
   });
-  std::vector<int4> ch;
-  bool runs = true;
-  int lo = 0, hi = -1, most = 0;  // the open chunk's entries
-  unsigned first = 0;
-  auto close = [&](unsigned end) {
-    if (end > first) {
-      const int n = hi >= lo ? hi - lo + 1 : 0;
-      ch.push_back(make_int4((int)first, (int)(end - first), n ? lo : 0, n));
-      most = std::max(most, n);
-    }
-    first = end;
-    lo = 0;
-    hi = -1;
-  };
-  for (size_t s = 0; s < (size_t)n_sl && runs; s++) {
-    const int l = span[s].x, h = span[s].y;
-    runs = h < l || h - l < kMost;
-    if (h < l)
-      continue;  // (padding alone joins the open chunk)
-    if (hi >= lo && std::max(hi, h) - std::min(lo, l) >= kFull)
-      close(slice_begin[s]);
-    lo = hi >= lo ? std::min(lo, l) : l;
-    hi = std::max(hi, h);
-  }
-  if (runs)
-    close(slice_begin.back());
-  if (runs && !ch.empty()) {
+  const std::vector<SlotChunk> ch = slot_chunks(slice_begin, span);
+  if (!ch.empty()) {
     std::vector<unsigned short> ix((size_t)n_slots, 0xffffu);
     parallel_for((long long)ch.size(), [&](long long a, long long b) {
       for (long long q = a; q < b; q++) {
-        const int4 c = ch[(size_t)q];
-        for (int i = 0; i < c.y; i++)
-          if (in[(size_t)c.x + i] >= 0)
-            ix[(size_t)c.x + i] = (unsigned short)(in[(size_t)c.x + i] - c.z);
+        const SlotChunk c = ch[(size_t)q];
+        for (size_t p = c.first, end = p + c.slots; p < end; p++)
+          if (in[p] >= 0)
+            ix[p] = (unsigned short)(in[p] - c.entry);
       }
     });
-    ISPM_CUDA_TRY(cudaMalloc(&chunk, ch.size() * sizeof(int4)));
-    ISPM_CUDA_TRY(cudaMemcpy(chunk, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    ISPM_CUDA_TRY(cudaMalloc(&chunk, ch.size() * sizeof(SlotChunk)));
+    ISPM_CUDA_TRY(
+        cudaMemcpy(chunk, ch.data(), ch.size() * sizeof(SlotChunk), cudaMemcpyHostToDevice));
     ISPM_CUDA_TRY(cudaMalloc(&idx, ix.size() * sizeof(unsigned short)));
     ISPM_CUDA_TRY(
         cudaMemcpy(idx, ix.data(), ix.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
     n_chunks = (int)ch.size();
-    max_entries = most;
+    for (const SlotChunk &c : ch)
+      max_entries = std::max(max_entries, c.entries);
     return ISPM_OK;
   }
   ISPM_CUDA_TRY(cudaMalloc(&inv, std::max<size_t>(in.size(), 1) * sizeof(int)));
@@ -539,7 +555,7 @@ int refresh_slots_t(E *elms, E2 *second, const SlotMap &m, const V *vals, const 
                          : cudaSuccess;
     if (e == cudaSuccess)
       e = launch_kernel(kernel, dim3(m.n_chunks), dim3(256), smem, s, true, elms, second,
-                        (const int4 *)m.chunk, (const unsigned short *)m.idx, vals, amax);
+                        (const SlotChunk *)m.chunk, (const unsigned short *)m.idx, vals, amax);
   } else {
     const long long blocks =
         std::min<long long>((m.n_slots + 255) / 256, (long long)device_sm_count() * 16);
@@ -744,6 +760,27 @@ int ispm_get_device_string(char *buf, int len)
   snprintf(buf, (size_t)len, "%04x:%02x:%02x (%s)", p.pciDomainID, p.pciBusID, p.pciDeviceID,
            p.name);
   return ISPM_OK;
+}
+
+int ispm_refresh_chunks(int n_slices, const unsigned *slice_begin, const int *first_entry,
+                        const int *last_entry, ispm_refresh_chunk *out, int cap)
+{
+  clear_error();
+  if (n_slices < 0 || !slice_begin || (n_slices && (!first_entry || !last_entry)) ||
+      (cap > 0 && !out))
+    return -1;
+  try {
+    std::vector<int2> span;
+    for (int s = 0; s < n_slices; s++)
+      span.push_back(make_int2(first_entry[s], last_entry[s]));
+    const std::vector<SlotChunk> ch =
+        slot_chunks(std::vector<unsigned>(slice_begin, slice_begin + n_slices + 1), span);
+    for (size_t k = 0; k < ch.size() && (int)k < cap; k++)
+      out[k] = ispm_refresh_chunk{ch[k].first, ch[k].slots, ch[k].entry, ch[k].entries};
+    return (int)ch.size();
+  } catch (const std::bad_alloc &) {
+    return -1;
+  }
 }
 
 int ispm_dslell_upload(const ispm_slell *h, ispm_dslell **out)

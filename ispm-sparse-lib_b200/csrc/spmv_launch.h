@@ -194,8 +194,17 @@ int refresh_values(DeviceSlell &d, const unsigned *map, const void *vals, int va
 // reads and writes are whole lines and a slot costs 2 bytes of map.  A shape
 // whose slices do not cover short runs (a transposed factor) keeps the entry
 // of each slot instead and gathers.
+struct SlotChunk {
+  unsigned first, slots;  // (a matrix may have up to 2^32 - 1 slots)
+  int entry, entries;     // first entry, entries
+};
+// The chunks of slices that start at slots slice_begin[0 .. n] and hold
+// entries span[s].x .. span[s].y (x > y: padding alone), or none where a slice
+// covers too long a run for a chunk.
+std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
+                                   const std::vector<int2> &span);
 struct SlotMap {
-  int4 *chunk = nullptr;          // first slot, slots, first entry, entries
+  SlotChunk *chunk = nullptr;
   unsigned short *idx = nullptr;  // slot -> entry within its chunk (0xffff: padding)
   int *inv = nullptr;             // slot -> entry (-1: padding), when not in chunks
   int n_chunks = 0, max_entries = 0;
