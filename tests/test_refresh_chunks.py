@@ -27,7 +27,7 @@ def chunks(ispm, begin, lo, hi):
 def check(ch, begin, lo, hi):
     at = 0
     for first, slots, entry, entries in ch:
-        assert first == at and 0 < slots < 2**31
+        assert first == at and 0 < slots <= 8192
         at += slots
         # the slices whose slots it holds
         a = np.searchsorted(begin, first, side="right") - 1
@@ -40,9 +40,9 @@ def check(ch, begin, lo, hi):
     assert at == begin[-1]
 
 
-@pytest.mark.parametrize("slots,count", [(1 << 20, 4000), (1 << 10, 700), (3, 50)])
+@pytest.mark.parametrize("slots,count", [(1 << 20, 2300), (1 << 10, 700), (3, 50)])
 def test_chunks_cover_every_slot(ispm, slots, count):
-    begin = np.arange(count + 1, dtype=np.int64) * slots  # 4.19e9 slots in the first case
+    begin = np.arange(count + 1, dtype=np.int64) * slots  # 2.4e9 slots in the first case
     width = min(slots, 900)
     lo = np.arange(count) * width
     hi = lo + width - 1
@@ -55,3 +55,12 @@ def test_long_slices_and_no_slices(ispm):
     assert chunks(ispm, begin, [0, 5, 20], [4, 5 + 8192, 30]) == []  # gathered
     assert len(chunks(ispm, begin, [0, 5, 20], [4, 5 + 8191, 30])) >= 1
     assert chunks(ispm, np.array([0]), [], []) == []
+    # a taller slice among many short runs: gathered; most of them tall: chunks
+    begin = np.arange(101) * 6000
+    for every, form in ((10, False), (1, True)):
+        width = np.where(np.arange(100) % every == 0, 6000, 2000)
+        hi = np.cumsum(width)
+        ch = chunks(ispm, begin, hi - width, hi - 1)
+        assert bool(ch) == form
+        if ch:
+            check(ch, begin, hi - width, hi - 1)
