@@ -454,6 +454,8 @@ void SlotMap::release()
   n_slots = 0;
 }
 
+constexpr int kChunkEntries = 8192;  // the most entries of a chunk
+
 std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
                                    const std::vector<int2> &span)
 {
@@ -464,7 +466,7 @@ std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
   // the entries again (a long row among short ones makes a slice of mostly
   // padding).  FP64, 200,000 rows of 5 entries with every 2,000th of 8,000: 25.4
   // us a refresh with neither rule, 15.6 split, 11.2 gathered.
-  constexpr int kFull = 3072, kMost = 8192;
+  constexpr int kFull = 3072;
   constexpr unsigned kSlots = 8192;
   std::vector<SlotChunk> ch;
   size_t tall = 0, runs = 0;
@@ -486,7 +488,7 @@ std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
     const int l = span[s].x, h = span[s].y;
     if (h < l)
       continue;  // (padding alone joins the open chunk)
-    if (h - l >= kMost)
+    if (h - l >= kChunkEntries)
       return {};
     if (hi >= lo && std::max(hi, h) - std::min(lo, l) >= kFull)
       close(slice_begin[s]);
@@ -559,8 +561,9 @@ int refresh_slots_t(E *elms, E2 *second, const SlotMap &m, const V *vals, const 
   if (m.chunk) {
     const size_t smem = (size_t)m.max_entries * sizeof(V);
     const auto kernel = refresh_chunks_kernel<E, E2, V>;
+    // (one limit for every map: another thread may be about to launch a larger one)
     e = smem > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)smem)
+                                                kChunkEntries * (int)sizeof(V))
                          : cudaSuccess;
     if (e == cudaSuccess)
       e = launch_kernel(kernel, dim3(m.n_chunks), dim3(256), smem, s, true, elms, second,
