@@ -501,6 +501,20 @@ std::vector<SlotChunk> slot_chunks(const std::vector<unsigned> &slice_begin,
   return ch;
 }
 
+// A map's device array; no memory leaves no error behind for later launches.
+template <class T> static int map_array(T **d, const T *h, size_t count)
+{
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  if (cudaMalloc(d, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    *d = nullptr;
+    return fail(ISPM_ERR_NOMEM, "value refresh map: cudaMalloc(%zu)", bytes);
+  }
+  if (count)
+    ISPM_CUDA_TRY(cudaMemcpy(*d, h, count * sizeof(T), cudaMemcpyHostToDevice));
+  return ISPM_OK;
+}
+
 int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<unsigned> &pos)
 {
   release();
@@ -534,21 +548,19 @@ int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<u
             ix[p] = (unsigned short)(in[p] - c.entry);
       }
     });
-    ISPM_CUDA_TRY(cudaMalloc(&chunk, ch.size() * sizeof(SlotChunk)));
-    ISPM_CUDA_TRY(
-        cudaMemcpy(chunk, ch.data(), ch.size() * sizeof(SlotChunk), cudaMemcpyHostToDevice));
-    ISPM_CUDA_TRY(cudaMalloc(&idx, ix.size() * sizeof(unsigned short)));
-    ISPM_CUDA_TRY(
-        cudaMemcpy(idx, ix.data(), ix.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+    int e = map_array(&chunk, ch.data(), ch.size());
+    if (!e)
+      e = map_array(&idx, ix.data(), ix.size());
+    if (e) {
+      release();
+      return e;
+    }
     n_chunks = (int)ch.size();
     for (const SlotChunk &c : ch)
       max_entries = std::max(max_entries, c.entries);
     return ISPM_OK;
   }
-  ISPM_CUDA_TRY(cudaMalloc(&inv, std::max<size_t>(in.size(), 1) * sizeof(int)));
-  if (!in.empty())
-    ISPM_CUDA_TRY(cudaMemcpy(inv, in.data(), in.size() * sizeof(int), cudaMemcpyHostToDevice));
-  return ISPM_OK;
+  return map_array(&inv, in.data(), in.size());
 }
 
 namespace {
