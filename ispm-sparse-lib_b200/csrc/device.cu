@@ -358,6 +358,10 @@ __device__ __forceinline__ double f16_scale(const double *amax)
   return m > 0.0 ? scalbn(1.0, isfinite(m) ? 13 - ilogb(m) : 14) : 1.0;
 }
 
+// A scale whose inverse FP32 holds; with another the elements stay as they are
+// and the caller, who reads *amax back, refuses the update.
+__device__ __forceinline__ bool f16_scale_ok(double s) { return s >= 0x1p-126 && s <= 0x1p126; }
+
 // Values through shared memory (SlotMap).  Bound by HBM: 8 bytes of value, 2
 // of map and the element a slot.  61 x 75 x 83 27-point FP64 (10.0 M entries):
 // 43 us (4.2 TB/s); gathering each slot's value from the CSR, 4 bytes of map a
@@ -383,6 +387,8 @@ __global__ void __launch_bounds__(256)
   for (int i = threadIdx.x; i < entries; i += 256)
     sm[i] = __ldcs(v + i);
   const double scale = f16_scale(amax);
+  if (!f16_scale_ok(scale))
+    return;
   __syncthreads();
   auto value = [&](unsigned k) { return k == 0xffffu ? 0.0 : (double)sm[k]; };
   if (((c.x | c.y) & 3) == 0) {  // four slots a thread
@@ -422,6 +428,8 @@ __global__ void refresh_gather_kernel(E *__restrict__ elms, E2 *__restrict__ sec
 {
   pdl_wait();
   const double scale = f16_scale(amax);
+  if (!f16_scale_ok(scale))
+    return;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
     const int src = __ldcs(inv + k);

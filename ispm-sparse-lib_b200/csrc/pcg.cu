@@ -1197,7 +1197,8 @@ int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
   if (int e = fsai_build_values(S.n, f.max_pattern, f.a_rp, f.a_ci, a_v, f.g_rp, f.g_v, f.fb, 0))
     return e;
   // FP16: one power-of-two scale for both factors, formed on the device: the
-  // largest magnitude lands in [2^13, 2^14), below the binary16 maximum (65504)
+  // largest magnitude lands in [2^13, 2^14), below the binary16 maximum (65504);
+  // a scale out of FP32's range leaves both factors as they were
   const double *amax_d = f.f16 ? f.amax : nullptr;
   if (f.f16)
     if (int e = absmax_async(f.g_v, f.nnz_g, f.amax, 0))
@@ -1212,7 +1213,6 @@ int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
   } back;
   // (the count sits behind the maximum)
   ISPM_CUDA_TRY(cudaMemcpy(&back, f.amax, sizeof back, cudaMemcpyDeviceToHost));
-  S.fsai_fallbacks = back.fb[0];
   if (f.f16) {
     int ex = 0;
     if (back.amax > 0.0)
@@ -1222,6 +1222,7 @@ int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
       return fail(ISPM_ERR_INVALID, "FP16 factor: magnitudes out of the FP32 scale range");
     S.G.inv_scale = S.Ht.inv_scale = (float)(1.0 / sc);
   }
+  S.fsai_fallbacks = back.fb[0];
   return ISPM_OK;
 }
 

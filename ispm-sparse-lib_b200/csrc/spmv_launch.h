@@ -223,7 +223,8 @@ struct SlotMap {
 std::vector<unsigned> slice_begins(const HostSlell &h);
 // d.elms (and second->elms, of the same shape) = vals in the map's order, 0 on
 // padding.  amax (FP16 elements; device): values times the power of two that
-// maps *amax into [2^13, 2^14).
+// maps *amax into [2^13, 2^14); with one outside 2^-126 .. 2^126 nothing is
+// written.
 int refresh_slots(DeviceSlell &d, const SlotMap &map, const void *vals, int val_dtype,
                   cudaStream_t s, DeviceSlell *second = nullptr, const double *amax = nullptr);
 // *out = max |vals[k]| over n device values (device result; 0 for n = 0).
