@@ -1342,6 +1342,10 @@ int update_values(Solver &S, const double *vals, bool on_device)
   if (S.fsai_kept)
     if (int e = fsai_values(S, S.fsai, a_v))
       return e;
+  if (int e = S.refresh_persist())
+    return e;
+  // (a copy from pageable memory may return before it has landed, and the
+  // caller's next solve may be on a stream that does not wait for this one)
   ISPM_CUDA_TRY(cudaStreamSynchronize(0));
   // the iteration graph holds launch arguments by value (an FP16 factor's
   // scale among them): capture it again at the next solve
@@ -1349,7 +1353,7 @@ int update_values(Solver &S, const double *vals, bool on_device)
     cudaGraphExecDestroy(S.graph);
     S.graph = nullptr;
   }
-  return S.refresh_persist();
+  return ISPM_OK;
 }
 
 }  // namespace
@@ -1580,6 +1584,8 @@ int ispm_solver_create(int n, const int *row_ptr, const int *cols, const double 
   }
   if (int e = S.init_persist())
     return e;
+  // (the first solve may be on a stream that does not wait for this one)
+  ISPM_CUDA_TRY(cudaStreamSynchronize(0));
   *out = h.release();
   return ISPM_OK;
 }
