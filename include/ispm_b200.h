@@ -386,7 +386,8 @@ typedef struct {
                            node, repeated on the device until the flags end
                            the phase, so a phase is one graph launch and one
                            host wait; 0: eager launches.  A system small enough
-                           for L2 is solved in one launch, whatever this says */
+                           for L2 is solved in one launch, whatever this says
+                           (ispm_solver_set_one_launch) */
   double replace_ratio_f32; /* reliable update once the recursive residual fell by
                                this factor since the last one (FP32 inner) */
   double replace_ratio_f64; /* same for FP64 */
@@ -510,6 +511,16 @@ int ispm_solver_operator(const ispm_solver *s, int which, ispm_slell_view *view,
  * bytes do not show).  Host only. */
 int ispm_solver_choose_shape(int elm_dtype, int n, const int *row_ptr, const int *cols,
                              const double *vals, ispm_slell_params *out);
+/* Whether solves run as one cooperative launch on all SMs (1: the system's
+ * matrices and vectors stay in L2 and its shapes are ones that kernel walks) or
+ * as chunks of step kernels (0).  set: 0 keeps to the step kernels (use_graph
+ * and check_every then apply), 1 goes back; ISPM_ERR_INVALID where one launch
+ * is not possible.  Solves of several objects at once run one after another
+ * as one launch each and side by side as step kernels, which four threads
+ * with 64^3 27-point mixed systems are served faster by (5.3 against 7.2 ms a
+ * solve; two threads 7.7 against 6.7; smaller systems: one launch). */
+int ispm_solver_one_launch(const ispm_solver *s);
+int ispm_solver_set_one_launch(ispm_solver *s, int on);
 /* True relative residual after each outer cycle of the last solve; returns
  * the count (writes at most cap values). */
 int ispm_solver_history(const ispm_solver *s, double *out, int cap);
@@ -560,6 +571,9 @@ int ispm_batch_solve(ispm_batch *b, const double *b_dev, double *x_dev,
  * in and out inside the call. */
 int ispm_batch_solve_host(ispm_batch *b, const double *const *b_host, double *const *x_host,
                           ispm_solve_stats *lane_stats, ispm_solve_stats *total, void *stream);
+/* As ispm_solver_one_launch / ispm_solver_set_one_launch, for a batch. */
+int ispm_batch_one_launch(const ispm_batch *b);
+int ispm_batch_set_one_launch(ispm_batch *b, int on);
 /* Kernels the last solve launched (graph replays counted per node). */
 int ispm_batch_launches(const ispm_batch *b);
 /* Rows of the stacked FSAI factor built as Jacobi rows. */

@@ -420,7 +420,7 @@ struct Batch {
   int launches = 0;  // kernels launched by the last solve (graph nodes counted)
   // one cooperative launch a solve (persist.cu) for batches that fit L2
   struct Persist {
-    bool on = false;
+    bool can = false, on = false;  // prepared; taken
     PersistParams prm;
     PersistKind kind;
     std::vector<int> order;  // lane of each slot
@@ -935,7 +935,7 @@ int Batch::init_persist()
   P.ru2 = ru * ru;
   P.max_iters = opts.max_iters;
   P.max_refinements = opts.max_refinements;
-  k.on = true;
+  k.can = k.on = true;
   return ISPM_OK;
 }
 
@@ -1409,6 +1409,19 @@ int ispm_batch_solve_host(ispm_batch *b, const double *const *b_host, double *co
 int ispm_batch_launches(const ispm_batch *b) { return b ? b->b.launches : 0; }
 
 unsigned ispm_batch_fsai_fallbacks(const ispm_batch *b) { return b ? b->b.fsai_fallbacks : 0; }
+
+int ispm_batch_one_launch(const ispm_batch *b) { return b && b->b.pk.on; }
+
+int ispm_batch_set_one_launch(ispm_batch *b, int on)
+{
+  clear_error();
+  if (!b)
+    return fail(ISPM_ERR_INVALID, "NULL batch");
+  if (on && !b->b.pk.can)
+    return fail(ISPM_ERR_INVALID, "not a batch one launch can solve");
+  b->b.pk.on = on != 0;
+  return ISPM_OK;
+}
 
 void ispm_batch_free(ispm_batch *b) { delete b; }
 

@@ -609,7 +609,7 @@ struct Solver {
   int replacements = 0, restarts = 0;
   // one cooperative launch a solve (persist.cu) for systems that fit L2
   struct Persist {
-    bool on = false;
+    bool can = false, on = false;  // prepared; taken
     PersistParams prm;
     PersistLane lane;
     PersistKind kind;
@@ -951,14 +951,14 @@ struct Solver {
     P.ru2 = ru * ru;
     P.max_iters = opts.max_iters;
     P.max_refinements = opts.max_refinements;
-    k.on = true;
+    k.can = k.on = true;
     return ISPM_OK;
   }
 
   // (after a value update: the FP16 factor's scale is part of the lane)
   int refresh_persist()
   {
-    if (!pk.on)
+    if (!pk.can)
       return ISPM_OK;
     pk.lane.G.inv_scale = G.inv_scale;
     pk.lane.Ht.inv_scale = Ht.inv_scale;
@@ -1673,6 +1673,19 @@ int ispm_solver_update_values(ispm_solver *s, const double *vals, int vals_on_de
   if (!s->s.refreshable)
     return fail(ISPM_ERR_INVALID, "the solver was created without opts.refresh");
   return update_values(s->s, vals, vals_on_device != 0);
+}
+
+int ispm_solver_one_launch(const ispm_solver *s) { return s && s->s.pk.on; }
+
+int ispm_solver_set_one_launch(ispm_solver *s, int on)
+{
+  clear_error();
+  if (!s)
+    return fail(ISPM_ERR_INVALID, "NULL solver");
+  if (on && !s->s.pk.can)
+    return fail(ISPM_ERR_INVALID, "not a solver one launch can solve");
+  s->s.pk.on = on != 0;
+  return ISPM_OK;
 }
 
 void ispm_solver_free(ispm_solver *s) { delete s; }

@@ -765,6 +765,8 @@ def _declare_solver():
     L.ispm_solver_history.restype = i
     L.ispm_solver_free.argtypes = [vp]
     L.ispm_solver_free.restype = None
+    L.ispm_solver_one_launch.argtypes = [vp]
+    L.ispm_solver_set_one_launch.argtypes = [vp, i]
     L.ispm_solver_update_values.argtypes = [vp, vp, i]
     L.ispm_solver_update_values.restype = i
     _SOLVER_DECLARED = True
@@ -835,6 +837,16 @@ class PCGSolver:
     @property
     def rows(self) -> int:
         return int(_lib().ispm_solver_rows(self._h))
+
+    @property
+    def one_launch(self) -> bool:
+        """Solves run as one cooperative launch (ispm_solver_one_launch); set False
+        to keep to chunks of step kernels, True to go back."""
+        return bool(_lib().ispm_solver_one_launch(self._h))
+
+    @one_launch.setter
+    def one_launch(self, on: bool):
+        _check(_lib().ispm_solver_set_one_launch(self._h, int(on)))
 
     def _finish(self, status, st):
         if status not in (OK, ERR_NOT_CONVERGED, ERR_BREAKDOWN):
@@ -990,6 +1002,8 @@ def _declare_batch():
     L.ispm_batch_solve.restype = i
     L.ispm_batch_solve_host.argtypes = [vp, vp, vp, vp, C.POINTER(solve_stats), vp]
     L.ispm_batch_solve_host.restype = i
+    L.ispm_batch_one_launch.argtypes = [vp]
+    L.ispm_batch_set_one_launch.argtypes = [vp, i]
     L.ispm_batch_launches.argtypes = [vp]
     L.ispm_batch_launches.restype = i
     L.ispm_batch_fsai_fallbacks.argtypes = [vp]
@@ -1069,6 +1083,16 @@ class BatchSolver:
         ln = (C.c_int * max(n, 1))()
         _lib().ispm_batch_groups(self._h, fm, ln, n)
         return [((fm[g].S, fm[g].H, fm[g].V, fm[g].D), ln[g]) for g in range(n)]
+
+    @property
+    def one_launch(self) -> bool:
+        """Solves run as one cooperative launch (ispm_batch_one_launch); set False
+        to keep to chunks of step kernels, True to go back."""
+        return bool(_lib().ispm_batch_one_launch(self._h))
+
+    @one_launch.setter
+    def one_launch(self, on: bool):
+        _check(_lib().ispm_batch_set_one_launch(self._h, int(on)))
 
     @property
     def launches(self) -> int:
