@@ -521,6 +521,11 @@ int ispm_solver_choose_shape(int elm_dtype, int n, const int *row_ptr, const int
  * solve; two threads 7.7 against 6.7; smaller systems: one launch). */
 int ispm_solver_one_launch(const ispm_solver *s);
 int ispm_solver_set_one_launch(ispm_solver *s, int on);
+/* The longest wait of a CTA of a one-launch solve, in clock cycles (negative:
+ * the default, about a second).  A solve whose wait runs out returns
+ * ISPM_ERR_TIMEOUT with that status in its stats (true_relres NaN) and x
+ * unfinished; the solver stays usable. */
+int ispm_solver_set_wait_limit(ispm_solver *s, long long cycles);
 /* True relative residual after each outer cycle of the last solve; returns
  * the count (writes at most cap values). */
 int ispm_solver_history(const ispm_solver *s, double *out, int cap);
@@ -574,6 +579,8 @@ int ispm_batch_solve_host(ispm_batch *b, const double *const *b_host, double *co
 /* As ispm_solver_one_launch / ispm_solver_set_one_launch, for a batch. */
 int ispm_batch_one_launch(const ispm_batch *b);
 int ispm_batch_set_one_launch(ispm_batch *b, int on);
+/* As ispm_solver_set_wait_limit (every lane's stats tell of the timeout). */
+int ispm_batch_set_wait_limit(ispm_batch *b, long long cycles);
 /* Kernels the last solve launched (graph replays counted per node). */
 int ispm_batch_launches(const ispm_batch *b);
 /* Rows of the stacked FSAI factor built as Jacobi rows. */

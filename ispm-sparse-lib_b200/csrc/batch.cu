@@ -762,8 +762,19 @@ struct Batch {
     refinements.assign(n, 0);
     restarts.assign(n, 0);
     status.assign(n, ISPM_OK);
-    if (int e = pk.on ? run_persistent(b, x, s) : run_chunks(b, x, s))
+    if (int e = pk.on ? run_persistent(b, x, s) : run_chunks(b, x, s)) {
+      if (e == ISPM_ERR_TIMEOUT) {
+        ispm_solve_stats o{};
+        o.status = e;
+        o.true_relres = NAN;
+        o.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        for (int L = 0; L < n && lane_stats; L++)
+          lane_stats[L] = o;
+        if (total)
+          *total = o;
+      }
       return e;
+    }
     int worst = ISPM_OK, max_it = 0, max_ref = 0, all_conv = 1;
     double max_rel = 0.0;
     for (int L = 0; L < n; L++) {
@@ -1420,6 +1431,15 @@ int ispm_batch_set_one_launch(ispm_batch *b, int on)
   if (on && !b->b.pk.can)
     return fail(ISPM_ERR_INVALID, "not a batch one launch can solve");
   b->b.pk.on = on != 0;
+  return ISPM_OK;
+}
+
+int ispm_batch_set_wait_limit(ispm_batch *b, long long cycles)
+{
+  clear_error();
+  if (!b)
+    return fail(ISPM_ERR_INVALID, "NULL batch");
+  b->b.pk.prm.wait_cycles = cycles < 0 ? kPersistWaitCycles : cycles;
   return ISPM_OK;
 }
 

@@ -979,8 +979,17 @@ struct Solver {
       return e;
     ISPM_CUDA_TRY(cudaMemcpyAsync(k.host, k.dev, kPkZero + kPkBack, cudaMemcpyDeviceToHost, s));
     ISPM_CUDA_TRY(cudaStreamSynchronize(s));
-    if (((const unsigned *)k.host)[0])
+    if (((const unsigned *)k.host)[0]) {
+      replacements = restarts = 0;
+      if (stats) {
+        *stats = ispm_solve_stats{};
+        stats->status = ISPM_ERR_TIMEOUT;
+        stats->true_relres = NAN;
+        stats->seconds =
+            std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      }
       return fail(ISPM_ERR_TIMEOUT, "persistent solve: a group of CTAs waited too long");
+    }
     const PersistOut &o = *(const PersistOut *)(k.host + kPkZero);
     const int kept = std::min(o.n_history, k.history_cap);
     history.resize((size_t)std::max(kept, 0));
@@ -1146,9 +1155,9 @@ struct Solver {
       if (!e)
         e = solve(b_perm, x_perm, stats, own);
       // x in the caller's order whenever solve() ran (a refused non-finite b
-      // leaves the zero iterate)
+      // leaves the zero iterate, a wait that ran out what there is)
       if (!e || e == ISPM_ERR_NOT_CONVERGED || e == ISPM_ERR_BREAKDOWN ||
-          e == ISPM_ERR_INVALID) {
+          e == ISPM_ERR_INVALID || e == ISPM_ERR_TIMEOUT) {
         cudaError_t me = cudaMemsetAsync(x, 0, (size_t)n_pad * sizeof(double), own);
         if (me == cudaSuccess)
           permute_out_kernel<<<grid_for(n), kThreads, 0, own>>>(x, x_perm, perm, n);
@@ -1685,6 +1694,15 @@ int ispm_solver_set_one_launch(ispm_solver *s, int on)
   if (on && !s->s.pk.can)
     return fail(ISPM_ERR_INVALID, "not a solver one launch can solve");
   s->s.pk.on = on != 0;
+  return ISPM_OK;
+}
+
+int ispm_solver_set_wait_limit(ispm_solver *s, long long cycles)
+{
+  clear_error();
+  if (!s)
+    return fail(ISPM_ERR_INVALID, "NULL solver");
+  s->s.pk.prm.wait_cycles = cycles < 0 ? kPersistWaitCycles : cycles;
   return ISPM_OK;
 }
 

@@ -22,8 +22,8 @@
 // consecutive rows a thread spend most instructions on realigning x windows,
 // which pays where HBM sets the pace).
 //
-// Waits are bounded: a CTA that has polled for kWaitCycles sets an abort flag
-// that every other wait sees, all CTAs return, and the host reports
+// Waits are bounded: a CTA that has polled for PersistParams::wait_cycles sets an
+// abort flag that every other wait sees, all CTAs return, and the host reports
 // ISPM_ERR_TIMEOUT.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -41,7 +41,6 @@
 namespace ispm {
 namespace {
 
-constexpr long long kWaitCycles = 2000000000LL;  // about a second
 constexpr int kSums = 3;
 
 // Matrix words: read once an iteration, kept out of L1 (x lives there).
@@ -326,10 +325,10 @@ template <int V, int LP, bool WIDE> struct Group {
         if (__all_sync(0xffffffffu, (int)(c - target) >= 0))
           break;
         const long long waited = clock64() - t0;
-        if (waited > kWaitCycles) {
+        if (waited > P.wait_cycles) {
           atomicExch(P.abort, 1u);
           good = 0;
-        } else if (waited > kWaitCycles / 1000) {
+        } else if (waited > P.wait_cycles / 1000) {
           unsigned stop;
           asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
                        : "=r"(stop)

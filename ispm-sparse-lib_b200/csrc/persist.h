@@ -60,6 +60,8 @@ struct PersistOut {
   int n_history, pad;
 };
 
+constexpr long long kPersistWaitCycles = 2000000000LL;  // about a second
+
 struct PersistParams {
   const PersistLane *lanes = nullptr;  // device; lanes of one group in a row
   const int *cta_lane = nullptr;       // CTA -> first lane of its group
@@ -82,6 +84,7 @@ struct PersistParams {
   int batch = 0;              // the batched solver's accounting of phases
   double tol = 0, ru2 = 0;
   int max_iters = 0, max_refinements = 0;
+  long long wait_cycles = kPersistWaitCycles;  // longest wait of a CTA
 };
 
 // The operator as PersistOp, or false when its shape is not one the kernel
