@@ -526,6 +526,11 @@ int ispm_solver_set_one_launch(ispm_solver *s, int on);
  * ISPM_ERR_TIMEOUT with that status in its stats (true_relres NaN) and x
  * unfinished; the solver stays usable. */
 int ispm_solver_set_wait_limit(ispm_solver *s, long long cycles);
+/* For tests: the next one-launch solve finds its launch returning this CUDA
+ * error, and nothing runs.  A launch that cannot be resident (a process with a
+ * part of the SMs) leaves the object to the step kernels for good; other errors
+ * fail the solve. */
+int ispm_solver_refuse_launch(ispm_solver *s, int cuda_error);
 /* True relative residual after each outer cycle of the last solve; returns
  * the count (writes at most cap values). */
 int ispm_solver_history(const ispm_solver *s, double *out, int cap);
@@ -581,6 +586,8 @@ int ispm_batch_one_launch(const ispm_batch *b);
 int ispm_batch_set_one_launch(ispm_batch *b, int on);
 /* As ispm_solver_set_wait_limit (every lane's stats tell of the timeout). */
 int ispm_batch_set_wait_limit(ispm_batch *b, long long cycles);
+/* As ispm_solver_refuse_launch. */
+int ispm_batch_refuse_launch(ispm_batch *b, int cuda_error);
 /* Kernels the last solve launched (graph replays counted per node). */
 int ispm_batch_launches(const ispm_batch *b);
 /* Rows of the stacked FSAI factor built as Jacobi rows. */

@@ -421,6 +421,7 @@ struct Batch {
   // one cooperative launch a solve (persist.cu) for batches that fit L2
   struct Persist {
     bool can = false, on = false;  // prepared; taken
+    cudaError_t fault = cudaSuccess;  // (a test's, for the next launch)
     PersistParams prm;
     PersistKind kind;
     std::vector<int> order;  // lane of each slot
@@ -629,15 +630,20 @@ struct Batch {
 
   int init_persist();
 
-  // The whole batch in one launch; fills the lane results.
-  int run_persistent(const double *b, double *x, cudaStream_t s)
+  // The whole batch in one launch; fills the lane results.  (refused: the step
+  // kernels take this solve and the object's later ones)
+  int run_persistent(const double *b, double *x, cudaStream_t s, bool &refused)
   {
     Persist &k = pk;
     k.prm.b = b;
     k.prm.x = x;
     ISPM_CUDA_TRY(cudaMemsetAsync(k.zero, 0, k.zero_bytes, s));
-    if (int e = persist_launch(k.prm, k.kind, k.ctas, k.threads, s))
-      return e;
+    const int launch = persist_launch(k.prm, k.kind, k.ctas, k.threads, s, k.fault, refused);
+    k.fault = cudaSuccess;
+    if (refused)
+      k.can = k.on = false;
+    if (launch || refused)
+      return launch;
     launches = 1;
     ISPM_CUDA_TRY(cudaMemcpyAsync(k.host, k.prm.out, sizeof(PersistOut) * n_lanes,
                                   cudaMemcpyDeviceToHost, s));
@@ -762,7 +768,11 @@ struct Batch {
     refinements.assign(n, 0);
     restarts.assign(n, 0);
     status.assign(n, ISPM_OK);
-    if (int e = pk.on ? run_persistent(b, x, s) : run_chunks(b, x, s)) {
+    bool steps = !pk.on;
+    int e = steps ? ISPM_OK : run_persistent(b, x, s, steps);
+    if (steps)
+      e = run_chunks(b, x, s);
+    if (e) {
       if (e == ISPM_ERR_TIMEOUT) {
         ispm_solve_stats o{};
         o.status = e;
@@ -1431,6 +1441,15 @@ int ispm_batch_set_one_launch(ispm_batch *b, int on)
   if (on && !b->b.pk.can)
     return fail(ISPM_ERR_INVALID, "not a batch one launch can solve");
   b->b.pk.on = on != 0;
+  return ISPM_OK;
+}
+
+int ispm_batch_refuse_launch(ispm_batch *b, int cuda_error)
+{
+  clear_error();
+  if (!b)
+    return fail(ISPM_ERR_INVALID, "NULL batch");
+  b->b.pk.fault = (cudaError_t)cuda_error;
   return ISPM_OK;
 }
 

@@ -610,6 +610,7 @@ struct Solver {
   // one cooperative launch a solve (persist.cu) for systems that fit L2
   struct Persist {
     bool can = false, on = false;  // prepared; taken
+    cudaError_t fault = cudaSuccess;  // (a test's, for the next launch)
     PersistParams prm;
     PersistLane lane;
     PersistKind kind;
@@ -967,7 +968,9 @@ struct Solver {
     return ISPM_OK;
   }
 
-  int solve_persistent(const double *b, double *x, ispm_solve_stats *stats, cudaStream_t s)
+  // (refused: the step kernels take this solve and the object's later ones)
+  int solve_persistent(const double *b, double *x, ispm_solve_stats *stats, cudaStream_t s,
+                       bool &refused)
   {
     auto t0 = std::chrono::steady_clock::now();
     history.clear();
@@ -975,8 +978,12 @@ struct Solver {
     k.prm.b = b;
     k.prm.x = x;
     ISPM_CUDA_TRY(cudaMemsetAsync(k.dev, 0, kPkZero, s));
-    if (int e = persist_launch(k.prm, k.kind, k.ctas, k.threads, s))
-      return e;
+    const int launch = persist_launch(k.prm, k.kind, k.ctas, k.threads, s, k.fault, refused);
+    k.fault = cudaSuccess;
+    if (refused)
+      k.can = k.on = false;
+    if (launch || refused)
+      return launch;
     ISPM_CUDA_TRY(cudaMemcpyAsync(k.host, k.dev, kPkZero + kPkBack, cudaMemcpyDeviceToHost, s));
     ISPM_CUDA_TRY(cudaStreamSynchronize(s));
     if (((const unsigned *)k.host)[0]) {
@@ -1022,8 +1029,12 @@ struct Solver {
 
   int solve(const double *b, double *x, ispm_solve_stats *stats, cudaStream_t s)
   {
-    if (pk.on)
-      return solve_persistent(b, x, stats, s);
+    if (pk.on) {
+      bool refused = false;
+      const int e = solve_persistent(b, x, stats, s, refused);
+      if (!refused)
+        return e;
+    }
     auto t0 = std::chrono::steady_clock::now();
     history.clear();
     replacements = restarts = 0;
@@ -1694,6 +1705,15 @@ int ispm_solver_set_one_launch(ispm_solver *s, int on)
   if (on && !s->s.pk.can)
     return fail(ISPM_ERR_INVALID, "not a solver one launch can solve");
   s->s.pk.on = on != 0;
+  return ISPM_OK;
+}
+
+int ispm_solver_refuse_launch(ispm_solver *s, int cuda_error)
+{
+  clear_error();
+  if (!s)
+    return fail(ISPM_ERR_INVALID, "NULL solver");
+  s->s.pk.fault = (cudaError_t)cuda_error;
   return ISPM_OK;
 }
 

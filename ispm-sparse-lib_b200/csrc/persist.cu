@@ -1101,7 +1101,7 @@ PersistShape persist_shape(double rows, double threads, double width, unsigned m
 }
 
 int persist_launch(const PersistParams &p, const PersistKind &k, int ctas, int threads,
-                   cudaStream_t s)
+                   cudaStream_t s, cudaError_t fault, bool &refused)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
@@ -1113,7 +1113,13 @@ int persist_launch(const PersistParams &p, const PersistKind &k, int ctas, int t
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, pick(k), p);
+  const cudaError_t e = fault != cudaSuccess ? fault : cudaLaunchKernelEx(&cfg, pick(k), p);
+  refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+            e == cudaErrorNotSupported;
+  if (refused) {
+    cudaGetLastError();
+    return ISPM_OK;
+  }
   return e == cudaSuccess ? ISPM_OK
                           : fail(ISPM_ERR_CUDA, "persistent solve: %s", cudaGetErrorString(e));
 }

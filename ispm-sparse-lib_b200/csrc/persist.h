@@ -101,9 +101,11 @@ constexpr size_t kPersistMaxSmem = 96 * 1024;  // (the rest of an SM's 228 KB is
 constexpr int kPersistParts = 6;
 constexpr int kPersistMaxDiag = 32;            // diagonals of a slice
 
-// One launch: cooperative, `ctas` CTAs of `threads` threads.
+// One launch: cooperative, `ctas` CTAs of `threads` threads.  refused (and
+// ISPM_OK, no launch and no error left): the CTAs cannot all be resident, where
+// the process has a part of the SMs.  fault: what a test has the launch return.
 int persist_launch(const PersistParams &p, const PersistKind &k, int ctas, int threads,
-                   cudaStream_t s);
+                   cudaStream_t s, cudaError_t fault, bool &refused);
 
 // CTAs for lanes of the given work: shares proportional to it, at least one
 // each, at most ctas in all and at most one per 32 rows; lanes beyond the
