@@ -810,10 +810,12 @@ __global__ void __launch_bounds__(2 * kFeatRows, 4)
     o[k] = words[k / (kFeat / 2) * (kFeatLd / 2) + k % (kFeat / 2)];
 }
 
+int max_train_grid() { return device_sm_count() * 2; }
+
 int train_grid(long long M)
 {
   const long long blocks = (M + kBlockRows - 1) / kBlockRows;
-  return (int)std::max(1LL, std::min(blocks, (long long)device_sm_count() * 2));
+  return (int)std::max(1LL, std::min(blocks, (long long)max_train_grid()));
 }
 
 // Forward: CTAs that stay resident walk the rows in strides.
@@ -845,17 +847,32 @@ int set_smem_attrs()
 
 struct ispm_mlp {
   float *prm = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr;
-  float *host = nullptr;  // pinned: results on their way to the caller (kPart floats)
   mutable std::mutex host_mu;
-  int part_cta = 0;
+  mutable std::vector<float> host;  // results on their way to the caller
+  mutable float *pinned = nullptr;
+  mutable int copies = 0;
+  // Where the next copy lands (host_mu held).  A pinned block saves a copy 5 us
+  // but costs the object 3 ms (2.6 to make, 0.5 to free), more than everything
+  // else a short-lived one does (0.4 ms to make, 0.1 its first step, 0.3 to
+  // free): it is made once the copies have cost as much without it.
+  float *landing() const
+  {
+    constexpr int kPinAfter = 600;
+    if (copies < kPinAfter && ++copies == kPinAfter &&
+        cudaMallocHost(&pinned, host.size() * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      pinned = nullptr;
+    }
+    return pinned ? pinned : host.data();
+  }
+  int part_cta = 0;  // CTAs that part has room for
   int step = 0;
   ~ispm_mlp()
   {
-    if (host)
-      cudaFreeHost(host);
-    for (float *p : {prm, m, v, grad, part})
-      if (p)
-        cudaFree(p);
+    if (pinned)
+      cudaFreeHost(pinned);
+    if (prm)
+      cudaFree(prm);  // (the others are parts of its block)
   }
 };
 
@@ -874,17 +891,27 @@ int ispm_mlp_create(const float *init_params, ispm_mlp **out)
   std::unique_ptr<ispm_mlp> h(new (std::nothrow) ispm_mlp);
   if (!h)
     return fail(ISPM_ERR_NOMEM, "host allocation");
-  for (float **pp : {&h->prm, &h->m, &h->v, &h->grad}) {
-    if (cudaMalloc(pp, sizeof(float) * kPart) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(ISPM_ERR_NOMEM, "cudaMalloc");
-    }
-    ISPM_CUDA_TRY(cudaMemset(*pp, 0, sizeof(float) * kPart));
-  }
-  ISPM_CUDA_TRY(cudaMemcpy(h->prm, init_params, sizeof(float) * kParams, cudaMemcpyHostToDevice));
-  if (cudaMallocHost(&h->host, sizeof(float) * kPart) != cudaSuccess) {
+  // one block for everything, the gradient's partials (of the most CTAs a step
+  // has) too: it takes no longer to make than the small arrays one by one, and
+  // no step allocates (a first one took 0.4 ms, 2.7 and more on a busy host)
+  constexpr size_t each = (kPart + 63) / 64 * 64;
+  h->part_cta = max_train_grid();
+  if (cudaMalloc(&h->prm, sizeof(float) * (4 * each + kPart * (size_t)h->part_cta)) !=
+      cudaSuccess) {
     cudaGetLastError();
-    return fail(ISPM_ERR_NOMEM, "pinned host allocation");
+    h->prm = nullptr;
+    return fail(ISPM_ERR_NOMEM, "cudaMalloc");
+  }
+  h->m = h->prm + each;
+  h->v = h->m + each;
+  h->grad = h->v + each;
+  h->part = h->grad + each;
+  ISPM_CUDA_TRY(cudaMemset(h->prm, 0, sizeof(float) * 4 * each));
+  ISPM_CUDA_TRY(cudaMemcpy(h->prm, init_params, sizeof(float) * kParams, cudaMemcpyHostToDevice));
+  try {
+    h->host.resize(kPart);
+  } catch (const std::bad_alloc &) {
+    return fail(ISPM_ERR_NOMEM, "host allocation");
   }
   if (int e = set_smem_attrs())
     return e;
@@ -898,9 +925,10 @@ int ispm_mlp_get_params(const ispm_mlp *m, float *host_out)
   if (!m || !host_out)
     return fail(ISPM_ERR_INVALID, "NULL argument");
   std::lock_guard<std::mutex> lock(m->host_mu);
-  ISPM_CUDA_TRY(cudaMemcpyAsync(m->host, m->prm, sizeof(float) * kParams, cudaMemcpyDeviceToHost, 0));
+  float *at = m->landing();
+  ISPM_CUDA_TRY(cudaMemcpyAsync(at, m->prm, sizeof(float) * kParams, cudaMemcpyDeviceToHost, 0));
   ISPM_CUDA_TRY(cudaStreamSynchronize(0));
-  memcpy(host_out, m->host, sizeof(float) * kParams);
+  memcpy(host_out, at, sizeof(float) * kParams);
   return ISPM_OK;
 }
 
@@ -944,17 +972,7 @@ int ispm_mlp_loss_grad(ispm_mlp *m, long long n_rows, const void *feat_bf16,
     return fail(ISPM_ERR_INVALID, "misaligned features / targets / weights");
   if (int e = set_smem_attrs())
     return e;
-  const int grid = train_grid(n_rows);
-  if (grid > m->part_cta) {
-    if (m->part)
-      cudaFree(m->part);
-    m->part = nullptr;
-    if (cudaMalloc(&m->part, sizeof(float) * kPart * grid) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(ISPM_ERR_NOMEM, "cudaMalloc");
-    }
-    m->part_cta = grid;
-  }
+  const int grid = std::min(train_grid(n_rows), m->part_cta);
   cudaStream_t s = (cudaStream_t)stream;
   // (programmatic launches: each kernel is set up while the one before it ends
   // and waits on the device for its results)
@@ -969,13 +987,14 @@ int ispm_mlp_loss_grad(ispm_mlp *m, long long n_rows, const void *feat_bf16,
   if (grad_out || loss_out) {  // one copy: the loss sits behind the gradient
     std::lock_guard<std::mutex> lock(m->host_mu);
     const size_t from = grad_out ? 0 : kParams;
-    ISPM_CUDA_TRY(cudaMemcpyAsync(m->host + from, m->grad + from, sizeof(float) * (kPart - from),
+    float *at = m->landing();
+    ISPM_CUDA_TRY(cudaMemcpyAsync(at + from, m->grad + from, sizeof(float) * (kPart - from),
                                   cudaMemcpyDeviceToHost, s));
     ISPM_CUDA_TRY(cudaStreamSynchronize(s));
     if (grad_out)
-      memcpy(grad_out, m->host, sizeof(float) * kParams);
+      memcpy(grad_out, at, sizeof(float) * kParams);
     if (loss_out)
-      *loss_out = m->host[kParams];
+      *loss_out = at[kParams];
   }
   return ISPM_OK;
 }
