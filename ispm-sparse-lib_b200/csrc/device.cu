@@ -6,8 +6,11 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "cuda_util.cuh"
@@ -441,6 +444,21 @@ __global__ void refresh_gather_kernel(E *__restrict__ elms, E2 *__restrict__ sec
   pdl_trigger();
 }
 
+template <class E>
+__global__ void scatter_values_kernel(E *__restrict__ elms, const unsigned *__restrict__ map,
+                                      const double *__restrict__ vals, long long n,
+                                      const double *amax)
+{
+  pdl_wait();
+  const double scale = f16_scale(amax);
+  if (!f16_scale_ok(scale))
+    return;
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x)
+    elms[__ldcs(map + k)] = element<E>(__ldg(vals + k), scale);
+  pdl_trigger();
+}
+
 std::vector<unsigned> slice_begins(const HostSlell &h)
 {
   const unsigned spe = 1 + (h.hblock > 1) + (h.var_height ? 1 : 0) + (h.diags ? 2 : 0);
@@ -527,38 +545,60 @@ int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<u
 {
   release();
   n_slots = slice_begin.back();
-  std::vector<int> in((size_t)n_slots, -1);
-  parallel_for((long long)pos.size(), [&](long long a, long long b) {
-    for (long long k = a; k < b; k++)
-      in[pos[(size_t)k]] = (int)k;
-  });
+  const size_t n = (size_t)n_slots;
+  // Host passes over entries and slots, 65,536 of them a thread at least (a
+  // thread's start-up costs as much); the pages of the arrays are first touched
+  // in them.  slot -> entry + 1 (0: padding)
+  constexpr long long kGrain = 65536;
+  struct Free {
+    void operator()(void *p) const { free(p); }
+  };
+  const std::unique_ptr<int[], Free> own((int *)calloc(std::max<size_t>(n, 1), sizeof(int)));
+  int *const in = own.get();
+  if (!in)
+    return fail(ISPM_ERR_NOMEM, "host allocation while mapping values");
+  parallel_for(
+      (long long)pos.size(),
+      [&](long long a, long long b) {
+        for (long long k = a; k < b; k++)
+          in[pos[(size_t)k]] = (int)k + 1;
+      },
+      kGrain);
+  const auto grain = [&](size_t parts) {
+    return std::max(1LL, (long long)(kGrain * (double)parts / std::max(1.0, (double)n)));
+  };
   const long long n_sl = (long long)slice_begin.size() - 1;
   std::vector<int2> span((size_t)n_sl);  // first and last entry of a slice
-  parallel_for(n_sl, [&](long long a, long long b) {
-    for (long long s = a; s < b; s++) {
-      int l = 0x7fffffff, h = -1;
-      for (unsigned p = slice_begin[s]; p < slice_begin[s + 1]; p++)
-        if (in[p] >= 0) {
-          l = std::min(l, in[p]);
-          h = std::max(h, in[p]);
+  parallel_for(
+      n_sl,
+      [&](long long a, long long b) {
+        for (long long s = a; s < b; s++) {
+          int l = 0x7fffffff, h = -1;
+          for (unsigned p = slice_begin[s]; p < slice_begin[s + 1]; p++)
+            if (in[p]) {
+              l = std::min(l, in[p] - 1);
+              h = std::max(h, in[p] - 1);
+            }
+          span[(size_t)s] = make_int2(l, h);
         }
-      span[(size_t)s] = make_int2(l, h);
-    }
-  });
+      },
+      grain((size_t)n_sl));
   const std::vector<SlotChunk> ch = slot_chunks(slice_begin, span);
   if (!ch.empty()) {
-    std::vector<unsigned short> ix((size_t)n_slots, 0xffffu);
-    parallel_for((long long)ch.size(), [&](long long a, long long b) {
-      for (long long q = a; q < b; q++) {
-        const SlotChunk c = ch[(size_t)q];
-        for (size_t p = c.first, end = p + c.slots; p < end; p++)
-          if (in[p] >= 0)
-            ix[p] = (unsigned short)(in[p] - c.entry);
-      }
-    });
+    const std::unique_ptr<unsigned short[]> ix(new unsigned short[n]);
+    parallel_for(
+        (long long)ch.size(),
+        [&](long long a, long long b) {
+          for (long long q = a; q < b; q++) {
+            const SlotChunk c = ch[(size_t)q];
+            for (size_t p = c.first, end = p + c.slots; p < end; p++)
+              ix[p] = in[p] ? (unsigned short)(in[p] - 1 - c.entry) : (unsigned short)0xffffu;
+          }
+        },
+        grain(ch.size()));
     int e = map_array(&chunk, ch.data(), ch.size());
     if (!e)
-      e = map_array(&idx, ix.data(), ix.size());
+      e = map_array(&idx, ix.get(), n);
     if (e) {
       release();
       return e;
@@ -568,7 +608,14 @@ int SlotMap::build(const std::vector<unsigned> &slice_begin, const std::vector<u
       max_entries = std::max(max_entries, c.entries);
     return ISPM_OK;
   }
-  return map_array(&inv, in.data(), in.size());
+  parallel_for(
+      n_slots,
+      [&](long long a, long long b) {
+        for (long long p = a; p < b; p++)
+          in[p]--;
+      },
+      kGrain);
+  return map_array(&inv, in, n);
 }
 
 namespace {
@@ -638,6 +685,30 @@ int refresh_slots(DeviceSlell &d, const SlotMap &map, const void *vals, int val_
   }
   return val_dtype == ISPM_F32 ? refresh_slots_v(d, map, (const float *)vals, amax, s)
                                : refresh_slots_v(d, map, (const double *)vals, amax, s);
+}
+
+int scatter_values(DeviceSlell &d, const unsigned *map, const double *vals, long long n,
+                   cudaStream_t s, const double *amax)
+{
+  if ((d.meta.elm_dtype == ISPM_F16) != (amax != nullptr))
+    return fail(ISPM_ERR_INVALID, "FP16 elements (alone) are refreshed with their scale");
+  if (!n)
+    return ISPM_OK;
+  const unsigned blocks =
+      (unsigned)std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8);
+  const auto launch = [&](auto *elms) {
+    using E = typename std::remove_pointer<decltype(elms)>::type;
+    return launch_kernel(scatter_values_kernel<E>, dim3(blocks), dim3(256), 0, s, true, elms, map,
+                         vals, n, amax);
+  };
+  cudaError_t e = d.meta.elm_dtype == ISPM_F64    ? launch((double *)d.elms)
+                  : d.meta.elm_dtype == ISPM_F32  ? launch((float *)d.elms)
+                  : d.meta.elm_dtype == ISPM_BF16 ? launch((__nv_bfloat16 *)d.elms)
+                                                  : launch((__half *)d.elms);
+  if (e == cudaSuccess)
+    e = cudaPeekAtLastError();
+  return e == cudaSuccess ? ISPM_OK
+                          : fail(ISPM_ERR_CUDA, "value scatter: %s", cudaGetErrorString(e));
 }
 
 // *out = max |v_k| as the bit pattern of a non-negative double (which orders

@@ -11,14 +11,15 @@
 
 namespace ispm {
 
-template <class F> void parallel_for(long long n, F fn)
+// grain: the fewest items a thread; below a few thousand of them the thread
+// start-up costs more than it saves.
+template <class F> void parallel_for(long long n, F fn, long long grain)
 {
   if (n <= 0)
     return;
   long long nt = host_threads();
-  // Below a few thousand items the thread start-up costs more than it saves.
-  if (nt > n / 2048)
-    nt = std::max(1LL, n / 2048);
+  if (nt > n / grain)
+    nt = std::max(1LL, n / grain);
   if (nt <= 1) {
     fn(0LL, n);
     return;

@@ -18,7 +18,7 @@ void clear_error();
 // Host worker pool size: ISPM_NUM_THREADS, else hardware concurrency.
 int host_threads();
 // Run fn(lo, hi) over [0, n) split into contiguous chunks on host threads.
-template <class F> void parallel_for(long long n, F fn);
+template <class F> void parallel_for(long long n, F fn, long long grain = 2048);
 
 // Host sliced-ELL matrix: the reference's slell_matrix<E, host>.
 struct HostSlell {

@@ -40,6 +40,7 @@
 
 #include "cuda_util.cuh"
 #include "fsai.h"
+#include "host_pool.h"
 #include "nvtx_range.h"
 #include "operator.h"
 #include "pcg_state.h"
@@ -586,7 +587,10 @@ struct Solver {
     int *a_rp = nullptr, *a_ci = nullptr, *g_rp = nullptr;
     unsigned *fb = nullptr;
     double *g_v = nullptr, *amax = nullptr;
-    std::shared_ptr<SlotMap> map_g, map_t;  // G's and G^T's slots from G's entries
+    // G's and G^T's slots from G's entries: maps where values come again, else
+    // G's entry -> slot
+    std::shared_ptr<SlotMap> map_g, map_t;
+    unsigned *pos_g = nullptr, *pos_t = nullptr;
     long long nnz_g = 0;
     int max_pattern = 0;
     bool f16 = false;
@@ -1223,10 +1227,13 @@ int fsai_values(Solver &S, const Solver::FsaiArrays &f, const double *a_v)
   if (f.f16)
     if (int e = absmax_async(f.g_v, f.nnz_g, f.amax, 0))
       return e;
-  if (int e = refresh_slots(S.G.dev, *f.map_g, f.g_v, ISPM_F64, 0, nullptr, amax_d))
-    return e;
-  if (int e = refresh_slots(S.Ht.dev, *f.map_t, f.g_v, ISPM_F64, 0, nullptr, amax_d))
-    return e;
+  for (int k = 0; k < 2; k++) {
+    DeviceSlell &d = k ? S.Ht.dev : S.G.dev;
+    const SlotMap *map = k ? f.map_t.get() : f.map_g.get();
+    if (int e = map ? refresh_slots(d, *map, f.g_v, ISPM_F64, 0, nullptr, amax_d)
+                    : scatter_values(d, k ? f.pos_t : f.pos_g, f.g_v, f.nnz_g, 0, amax_d))
+      return e;
+  }
   struct {
     double amax;
     unsigned fb[2];
@@ -1304,14 +1311,23 @@ int build_fsai_on_device(Solver &S, int n, const int *rp, const int *ci, const d
   }
   if (int e = to_device(mem, &f.g_rp, g_rp.data(), g_rp.size()))
     return e;
-  for (size_t k = 0; k < nnz_g; k++)  // G's entry -> slot of G^T
-    t_of[k] = pos_t[t_of[k]];
-  f.map_g = std::make_shared<SlotMap>();
-  f.map_t = std::make_shared<SlotMap>();
-  if (int e = f.map_g->build(begin_g, pos_g))
-    return e;
-  if (int e = f.map_t->build(begin_t, t_of))
-    return e;
+  parallel_for((long long)nnz_g, [&](long long a, long long b) {
+    for (long long k = a; k < b; k++)  // G's entry -> slot of G^T
+      t_of[k] = pos_t[t_of[k]];
+  }, 65536);
+  if (S.refreshable) {
+    f.map_g = std::make_shared<SlotMap>();
+    f.map_t = std::make_shared<SlotMap>();
+    if (int e = f.map_g->build(begin_g, pos_g))
+      return e;
+    if (int e = f.map_t->build(begin_t, t_of))
+      return e;
+  } else {
+    if (int e = to_device(mem, &f.pos_g, pos_g.data(), nnz_g))
+      return e;
+    if (int e = to_device(mem, &f.pos_t, t_of.data(), nnz_g))
+      return e;
+  }
   if (int e = mem.get(&f.g_v, nnz_g))
     return e;
   if (int e = mem.get(&f.amax, 2))
