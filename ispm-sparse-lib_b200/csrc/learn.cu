@@ -827,8 +827,12 @@ int fwd_grid(long long M)
 
 int set_smem_attrs()
 {
-  static std::atomic<bool> done{false};
-  if (done)
+  // (a kernel's limit is per device)
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  ISPM_CUDA_TRY(cudaGetDevice(&dev));
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load() & bit)
     return ISPM_OK;
   ISPM_CUDA_TRY(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(TrainSmem)));
@@ -838,7 +842,7 @@ int set_smem_attrs()
   ISPM_CUDA_TRY(cudaFuncSetAttribute(row_features_kernel<long long>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(FeatSmem)));
-  done = true;
+  done.fetch_or(bit);
   return ISPM_OK;
 }
 
