@@ -810,12 +810,10 @@ __global__ void __launch_bounds__(2 * kFeatRows, 4)
     o[k] = words[k / (kFeat / 2) * (kFeatLd / 2) + k % (kFeat / 2)];
 }
 
-int max_train_grid() { return device_sm_count() * 2; }
-
 int train_grid(long long M)
 {
   const long long blocks = (M + kBlockRows - 1) / kBlockRows;
-  return (int)std::max(1LL, std::min(blocks, (long long)max_train_grid()));
+  return (int)std::max(1LL, std::min(blocks, (long long)device_sm_count() * 2));
 }
 
 // Forward: CTAs that stay resident walk the rows in strides.
@@ -856,8 +854,8 @@ struct ispm_mlp {
   mutable float *pinned = nullptr;
   mutable int copies = 0;
   // Where the next copy lands (host_mu held).  A pinned block saves a copy 5 us
-  // but costs the object 3 ms (2.6 to make, 0.5 to free), more than everything
-  // else a short-lived one does (0.4 ms to make, 0.1 its first step, 0.3 to
+  // but costs a process's only object 3 ms (2.6 to make, 0.5 to free), more than
+  // all else a short-lived one does (0.4 ms to make, 0.4 its first step, 0.6 to
   // free): it is made once the copies have cost as much without it.
   float *landing() const
   {
@@ -869,14 +867,15 @@ struct ispm_mlp {
     }
     return pinned ? pinned : host.data();
   }
-  int part_cta = 0;  // CTAs that part has room for
+  int part_cta = 0;
   int step = 0;
   ~ispm_mlp()
   {
     if (pinned)
       cudaFreeHost(pinned);
-    if (prm)
-      cudaFree(prm);  // (the others are parts of its block)
+    for (float *p : {prm, part})  // (m, v and grad are in prm's block)
+      if (p)
+        cudaFree(p);
   }
 };
 
@@ -895,13 +894,10 @@ int ispm_mlp_create(const float *init_params, ispm_mlp **out)
   std::unique_ptr<ispm_mlp> h(new (std::nothrow) ispm_mlp);
   if (!h)
     return fail(ISPM_ERR_NOMEM, "host allocation");
-  // one block for everything, the gradient's partials (of the most CTAs a step
-  // has) too: it takes no longer to make than the small arrays one by one, and
-  // no step allocates (a first one took 0.4 ms, 2.7 and more on a busy host)
+  // (part, 7.7 MB, waits for a training step: with it an object takes 0.5 ms to
+  // make, not 0.1, which a prediction never needs)
   constexpr size_t each = (kPart + 63) / 64 * 64;
-  h->part_cta = max_train_grid();
-  if (cudaMalloc(&h->prm, sizeof(float) * (4 * each + kPart * (size_t)h->part_cta)) !=
-      cudaSuccess) {
+  if (cudaMalloc(&h->prm, sizeof(float) * 4 * each) != cudaSuccess) {
     cudaGetLastError();
     h->prm = nullptr;
     return fail(ISPM_ERR_NOMEM, "cudaMalloc");
@@ -909,7 +905,6 @@ int ispm_mlp_create(const float *init_params, ispm_mlp **out)
   h->m = h->prm + each;
   h->v = h->m + each;
   h->grad = h->v + each;
-  h->part = h->grad + each;
   ISPM_CUDA_TRY(cudaMemset(h->prm, 0, sizeof(float) * 4 * each));
   ISPM_CUDA_TRY(cudaMemcpy(h->prm, init_params, sizeof(float) * kParams, cudaMemcpyHostToDevice));
   try {
@@ -976,7 +971,19 @@ int ispm_mlp_loss_grad(ispm_mlp *m, long long n_rows, const void *feat_bf16,
     return fail(ISPM_ERR_INVALID, "misaligned features / targets / weights");
   if (int e = set_smem_attrs())
     return e;
-  const int grid = std::min(train_grid(n_rows), m->part_cta);
+  const int grid = train_grid(n_rows);
+  if (grid > m->part_cta) {
+    if (m->part)
+      cudaFree(m->part);
+    m->part = nullptr;
+    m->part_cta = 0;
+    if (cudaMalloc(&m->part, sizeof(float) * kPart * grid) != cudaSuccess) {
+      cudaGetLastError();
+      m->part = nullptr;
+      return fail(ISPM_ERR_NOMEM, "cudaMalloc");
+    }
+    m->part_cta = grid;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   // (programmatic launches: each kernel is set up while the one before it ends
   // and waits on the device for its results)
