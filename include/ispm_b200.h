@@ -432,11 +432,12 @@ typedef struct {
                            499 against 501 iterations, on a B200). */
   int refresh;          /* keep what ispm_solver_update_values needs to take new
                            values of A (same sparsity pattern) on the device:
-                           the CSR-entry -> element-slot maps of both device
-                           copies of A, the renumbering's entry map and, with
+                           where the slots of both device copies of A take
+                           their values, the renumbering's entry map and, with
                            prec = ISPM_PREC_FSAI_GPU, the factor's device
-                           patterns (about 20 bytes per entry of A and 32 per
-                           entry of G).  Not with matrix_f16. */
+                           patterns (about 14 bytes per entry of A, 26 in a
+                           renumbered solve, and 14 per entry of G).  Not with
+                           matrix_f16. */
 } ispm_solver_opts;
 
 #define ISPM_REORDER_NONE 0

@@ -11,10 +11,12 @@
 // another's rows.  The lanes of a batch have groups of their own, sized by
 // their work, and never wait for one another.
 //
-// What bounds it: a meeting of 148 CTAs costs about 2.2 us (the release waits
-// 0.8 us for the step's stores, the count is seen 1 us later, the sums take
-// 0.4 us), three a pipelined and five a classic iteration, and a step's loads
-// come from L2 in a few dependent rounds.  So a step's loads go out in blocks
+// What bounds it: a meeting costs about 1.7 us on 7-point 24^3 (the release waits
+// 0.6 us for the step's stores, the count is seen 0.6 us later, the others' sums
+// take 0.4) and 2.2 on 27-point 56^3, three a pipelined and five a classic
+// iteration: over half of a solve's cycles up to there.  Past it CTAs wait for
+// the slowest one's loads (3.5 us on 72^3).  A step's loads come from L2 in a few
+// dependent rounds.  So a step's loads go out in blocks
 // before the first is used, the slice headers stay in shared memory for the
 // whole solve, and a thread takes whole rows with lanes on consecutive ones:
 // a diagonal step is one element load, one x load and one multiply-add a row

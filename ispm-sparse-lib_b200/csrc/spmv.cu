@@ -817,7 +817,7 @@ int launch_te(const ispm_launch_params &p, const ispm_slell_view &m, const void 
   if constexpr (std::is_same<T, float>::value) {
     StageInfo si;
     if (staged_shape(ISPM_F32, p, m, x, si, a.st_slots, a.st_slot_bytes, a.st_x_off)) {
-      a.pdl = 0;  // it fetches elements before it waits for the kernel before it
+      a.pdl = 0;  // it fetches elements before it waits, and a refresh may come before it
       return launch_staged<E>(a, si, s);
     }
   }

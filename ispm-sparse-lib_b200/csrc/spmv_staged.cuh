@@ -14,8 +14,9 @@
 // each lane eight rows (t = lane + 32 j), reading every element and x value
 // from shared memory with conflict-free 32-bit loads, and hand the slot back
 // through a second mbarrier.  The element copies of the first slots go out
-// before the programmatic-launch wait (the matrix is final before the
-// previous kernel starts), the x copies after it.  The copy warps keep up to
+// before the programmatic-launch wait, which would be right only where the
+// matrix is final before the previous kernel starts; a value refresh may be that
+// kernel, so launches of this walk are plain ones.  The copy warps keep up to
 // `slots` tiles in flight, so the bytes in flight per SM are set by shared
 // memory, not by registers or warps.  (Measured on this walk: the bulk-copy
 // engine, cp.async.bulk, moves about 17 bytes per cycle per SM, and one

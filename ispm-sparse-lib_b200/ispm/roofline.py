@@ -103,13 +103,13 @@ def run(log=print):
             slell_bytes(H.view(), 4 if dt == np.float32 else 8))
         del D, H, x, y
 
-    # value refresh: new CSR values scattered into the device matrix
+    # value refresh: new CSR values dealt out to the device matrix's slots
     A32 = csr_matrix(n, n, A.row_ptr, A.cols, A.elms.astype(np.float32))
     plan = spmv_plan(A32, T=np.float32)
     vals = torch.from_numpy(A.elms).to(dev)
     plan_refresh_values(plan, A32, vals)  # builds the map once
     add("value refresh (C2, FP64 -> FP32 slots)", timed(lambda: plan_refresh_values(plan, A32, vals)),
-        nnz * (8 + 4 + 4))
+        nnz * (8 + 2 + 4))  # value, its place in the chunk, element
     del plan, vals
 
     # BLAS
