@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 8
   for (int i = threadIdx.x; i < entries; i += 256)
     sm[i] = __ldcs(v + i);
-  const double scale = f16_scale(amax);
-  if (!f16_scale_ok(scale))
+  const double scale = std::is_same<E, __half>::value ? f16_scale(amax) : 1.0;
+  if (std::is_same<E, __half>::value && !f16_scale_ok(scale))
     return;
   __syncthreads();
   auto value = [&](unsigned k) { return k == 0xffffu ? 0.0 : (double)sm[k]; };
@@ -430,8 +430,8 @@ __global__ void refresh_gather_kernel(E *__restrict__ elms, E2 *__restrict__ sec
                                       long long n, const double *amax)
 {
   pdl_wait();
-  const double scale = f16_scale(amax);
-  if (!f16_scale_ok(scale))
+  const double scale = std::is_same<E, __half>::value ? f16_scale(amax) : 1.0;
+  if (std::is_same<E, __half>::value && !f16_scale_ok(scale))
     return;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
@@ -450,8 +450,8 @@ __global__ void scatter_values_kernel(E *__restrict__ elms, const unsigned *__re
                                       const double *amax)
 {
   pdl_wait();
-  const double scale = f16_scale(amax);
-  if (!f16_scale_ok(scale))
+  const double scale = std::is_same<E, __half>::value ? f16_scale(amax) : 1.0;
+  if (std::is_same<E, __half>::value && !f16_scale_ok(scale))
     return;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x)
