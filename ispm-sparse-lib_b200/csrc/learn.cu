@@ -860,10 +860,15 @@ struct ispm_mlp {
   float *landing() const
   {
     constexpr int kPinAfter = 600;
-    if (copies < kPinAfter && ++copies == kPinAfter &&
-        cudaMallocHost(&pinned, host.size() * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      pinned = nullptr;
+    if (copies < kPinAfter && ++copies == kPinAfter) {
+      // (another thread may be capturing a graph, which an allocation must not end)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (cudaMallocHost(&pinned, host.size() * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        pinned = nullptr;
+      }
+      cudaThreadExchangeStreamCaptureMode(&mode);
     }
     return pinned ? pinned : host.data();
   }
